@@ -1265,19 +1265,12 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 // 3-D map over planes [nsplit][rows][kpad] of 16-bit parts; box {bk, box_rows, 1}.
 int make_plane_map(CUtensorMap *map, const void *base, int64_t rows, int64_t kpad, int nsplit,
                    int box_rows, int bk, bool f16) {
-  auto fn = encode_fn();
-  if (!fn) return fail(GT_ECUDA, "cuTensorMapEncodeTiled unavailable");
-  cuuint64_t dims[3] = {cuuint64_t(kpad), cuuint64_t(rows), cuuint64_t(nsplit)};
-  cuuint64_t strides[2] = {cuuint64_t(kpad * 2), cuuint64_t(rows * kpad * 2)};
-  cuuint32_t box[3] = {cuuint32_t(bk), cuuint32_t(box_rows), 1u};
-  cuuint32_t estr[3] = {1u, 1u, 1u};
-  CUresult r = fn(map, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3,
-                  const_cast<void *>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  bk == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return fail(GT_ECUDA, "cuTensorMapEncodeTiled failed (%d)", int(r));
-  return GT_OK;
+  const cuuint64_t dims[3] = {cuuint64_t(kpad), cuuint64_t(rows), cuuint64_t(nsplit)};
+  const cuuint64_t strides[2] = {cuuint64_t(kpad * 2), cuuint64_t(rows * kpad * 2)};
+  const cuuint32_t box[3] = {cuuint32_t(bk), cuuint32_t(box_rows), 1u};
+  return tc_map_3d(map, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
+                   base, dims, strides, box,
+                   bk == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
 // Launches the persistent kernel over `ntiles` tiles of work source w.
@@ -1361,6 +1354,19 @@ int check_kind(int kind) {
 int kind_nsplit(int kind) { return kind == tc::KIND_BF16X6 ? 3 : 2; }
 
 }  // namespace
+
+int tc_map_3d(CUtensorMap *map, CUtensorMapDataType type, const void *base,
+              const cuuint64_t (&dims)[3], const cuuint64_t (&strides)[2],
+              const cuuint32_t (&box)[3], CUtensorMapSwizzle swizzle) {
+  auto fn = encode_fn();
+  if (!fn) return fail(GT_ECUDA, "cuTensorMapEncodeTiled unavailable");
+  const cuuint32_t estr[3] = {1u, 1u, 1u};
+  const CUresult r = fn(map, type, 3, const_cast<void *>(base), dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(GT_ECUDA, "cuTensorMapEncodeTiled failed (%d)", int(r));
+  return GT_OK;
+}
 
 int tc_plane_map(CUtensorMap *map, const void *base, int64_t rows, int64_t kpad, int nplanes,
                  int box_rows, int bk, bool f16) {

@@ -28,6 +28,11 @@ int euclid_tc(const float *d_pts, int64_t n, int64_t dim, float *d_out, int layo
 int tc_plane_map(CUtensorMap *map, const void *base, int64_t rows, int64_t kpad, int nplanes,
                  int box_rows, int bk, bool f16);
 
+// gram_tc.cu: any 3-D tensor map of dense boxes (no interleave, zero fill).
+int tc_map_3d(CUtensorMap *map, CUtensorMapDataType type, const void *base,
+              const cuuint64_t (&dims)[3], const cuuint64_t (&strides)[2],
+              const cuuint32_t (&box)[3], CUtensorMapSwizzle swizzle);
+
 // Per-variable statistics of the Pearson prologue.
 struct ColStats {
   double mean;

@@ -187,6 +187,17 @@ __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint6
       : "memory");
 }
 
+// The same with 8-bit operands (kind::f8f6f4, K = 32 elements per instruction).
+__device__ __forceinline__ void umma_f8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
+                                        uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
 // Arrive on `bar` once every tcgen05 operation issued so far by this thread
 // has completed.
 __device__ __forceinline__ void umma_commit(uint64_t *bar) {
@@ -281,6 +292,13 @@ __host__ __device__ constexpr uint32_t idesc_f32acc(int M, int N, uint32_t ab_fm
   return (1u << 4)                    // D format f32
          | (ab_fmt << 7)              // A format
          | (ab_fmt << 10)             // B format
+         | (uint32_t(N >> 3) << 17)   // N / 8
+         | (uint32_t(M >> 4) << 24);  // M / 16
+}
+
+// Instruction descriptor: kind::f8f6f4, D = f32, A and B K-major e4m3.
+__host__ __device__ constexpr uint32_t idesc_e4m3_f32acc(int M, int N) {
+  return (1u << 4)                    // D format f32; A and B format e4m3 = 0
          | (uint32_t(N >> 3) << 17)   // N / 8
          | (uint32_t(M >> 4) << 24);  // M / 16
 }
