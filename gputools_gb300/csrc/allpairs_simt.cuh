@@ -138,6 +138,68 @@ struct HasStagedMirror<T, std::void_t<decltype(T::kStagedMirror)>>
 template <int TM, int TN, int NACC>
 constexpr int simt_min_blocks() { return TM * TN * NACC <= 64 ? 2 : 1; }
 
+// Writes a tile's entries (and mirror) from the accumulators; T is the operand
+// buffer, idle by now (every thread has passed the main loop's last barrier).
+template <class Out, int TM, int TN, int NA>
+__device__ __forceinline__ void simt_write_tile(const SimtArgs &a, const Out &out, int ti, int tj,
+                                                int64_t row0, int64_t col0, float *T,
+                                                float (&acc)[TM][TN][NA]) {
+  constexpr int BM = 16 * TM, BN = 16 * TN, LDA = simt_ld<BM>();
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const bool mirror = a.symmetric && ti != tj;
+  if constexpr (HasStagedMirror<Out>::value) {
+    if (out.staged(mirror)) {
+      // the tile's entries, then its mirror in 32-row chunks through the
+      // (now idle) operand buffers: each warp writes 32 consecutive floats of
+      // a mirrored row per store
+      constexpr int kLdT = BN + 1;
+      static_assert(32 * kLdT <= 2 * kSimtBK * LDA, "a 32-row chunk fits the operand buffers");
+#pragma unroll
+      for (int i = 0; i < TM; i++) {
+        const int64_t r = row0 + simt_row(i, ty);
+#pragma unroll
+        for (int j = 0; j < TN; j++) {
+          const int64_t c = col0 + tx + 16 * j;
+          const float v = out.value(r, c, acc[i][j]);
+          acc[i][j][0] = v;
+          if (r < a.nr && c < a.nc) out.store(r, c, v);
+        }
+      }
+      const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+      for (int q = 0; q < BM / 32; q++) {
+        __syncthreads();  // the previous chunk (or the main loop) is done with T
+        // rows 32 q .. 32 q + 31: four rows of each thread of half the tile's ty
+#pragma unroll
+        for (int i = 0; i < TM; i++) {
+          const int lr = simt_row(i, ty) - 32 * q;
+          if (lr < 0 || lr >= 32) continue;
+#pragma unroll
+          for (int j = 0; j < TN; j++) T[lr * kLdT + tx + 16 * j] = acc[i][j][0];
+        }
+        __syncthreads();
+        const int64_t r = row0 + 32 * q + lane;
+        for (int cc = warp; cc < BN; cc += kSimtThreads / 32) {
+          const int64_t c = col0 + cc;
+          if (r < a.nr && c < a.nc) out.store(c, r, T[lane * kLdT + cc]);
+        }
+      }
+      return;
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < TM; i++) {
+    const int64_t r = row0 + simt_row(i, ty);
+    if (r >= a.nr) continue;
+#pragma unroll
+    for (int j = 0; j < TN; j++) {
+      const int64_t c = col0 + tx + 16 * j;
+      if (c >= a.nc) continue;
+      out(r, c, acc[i][j], mirror);
+    }
+  }
+}
+
 template <class Op, class Out, int TM, int TN>
 __global__ void __launch_bounds__(kSimtThreads, simt_min_blocks<TM, TN, Op::NACC>())
 allpairs_simt_kernel(SimtArgs a, Op op, Out out) {
@@ -211,59 +273,7 @@ allpairs_simt_kernel(SimtArgs a, Op op, Out out) {
     __syncthreads();
   }
 
-  const bool mirror = a.symmetric && ti != tj;
-  if constexpr (HasStagedMirror<Out>::value) {
-    if (out.staged(mirror)) {
-      // the tile's entries, then its mirror in 32-row chunks through the
-      // (now idle) operand buffers: each warp writes 32 consecutive floats of
-      // a mirrored row per store
-      constexpr int kLdT = BN + 1;
-      static_assert(32 * kLdT <= 2 * kSimtBK * LDA, "a 32-row chunk fits the operand buffers");
-      float *T = &sA[0][0];
-#pragma unroll
-      for (int i = 0; i < TM; i++) {
-        const int64_t r = row0 + simt_row(i, ty);
-#pragma unroll
-        for (int j = 0; j < TN; j++) {
-          const int64_t c = col0 + tx + 16 * j;
-          const float v = out.value(r, c, acc[i][j]);
-          acc[i][j][0] = v;
-          if (r < a.nr && c < a.nc) out.store(r, c, v);
-        }
-      }
-      const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-      for (int q = 0; q < BM / 32; q++) {
-        __syncthreads();  // the previous chunk (or the main loop) is done with T
-        // rows 32 q .. 32 q + 31: four rows of each thread of half the tile's ty
-#pragma unroll
-        for (int i = 0; i < TM; i++) {
-          const int lr = simt_row(i, ty) - 32 * q;
-          if (lr < 0 || lr >= 32) continue;
-#pragma unroll
-          for (int j = 0; j < TN; j++) T[lr * kLdT + tx + 16 * j] = acc[i][j][0];
-        }
-        __syncthreads();
-        const int64_t r = row0 + 32 * q + lane;
-        for (int cc = warp; cc < BN; cc += kSimtThreads / 32) {
-          const int64_t c = col0 + cc;
-          if (r < a.nr && c < a.nc) out.store(c, r, T[lane * kLdT + cc]);
-        }
-      }
-      return;
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < TM; i++) {
-    const int64_t r = row0 + simt_row(i, ty);
-    if (r >= a.nr) continue;
-#pragma unroll
-    for (int j = 0; j < TN; j++) {
-      const int64_t c = col0 + tx + 16 * j;
-      if (c >= a.nc) continue;
-      out(r, c, acc[i][j], mirror);
-    }
-  }
+  simt_write_tile<Out, TM, TN, NA>(a, out, ti, tj, row0, col0, &sA[0][0], acc);
 }
 
 template <class Op, class Out, int TM, int TN>
