@@ -466,14 +466,14 @@ struct EuclidLineFinish {
   }
 };
 
-// B-spline mutual information (inst/cuda/mi.cu:115-152 get_mi): rows and
-// columns are (variable, bin) with 2^lg bins per variable (zero padded), the
-// Gram entry times gscale / nsamples is the joint probability p_ab of the
-// two variables' bins.  A 32 x 32 block holds whole bin blocks: each lane sums
-// p log2 p over a column variable's bins, the lanes of one row variable add
-// their sums, and MI = that sum + H(x) + H(y) goes to out[y * ldo + x] (the
+// Mutual information (gpuMi): the operand rows are B-spline weights, 32 / S
+// variables to a group of 32 rows, S rows each (the bins, then zero rows), so
+// a 32 x 32 block holds whole bin blocks and a Gram entry times gscale /
+// nsamples is the joint probability p_ab of the two variables' bins.  Each lane
+// sums p log2 p over a column variable's bins, the lanes of one row variable
+// add their sums, and MI = that sum + H(x) + H(y) goes to out[y * ldo + x] (the
 // reference layout; with symmetric, pairs x <= y and their mirror).
-template <int LG>  // log2 of the bins per variable: a compact body per bin count
+template <int S>  // rows per variable: a compact body per row count
 struct MiFinish {
   float *out;
   const float *hx, *hy;  // entropies of the row and column variables
@@ -481,37 +481,51 @@ struct MiFinish {
   float pscale;          // gscale / nsamples
   int symmetric;
   unsigned colmask;      // bit j: column j of a 32-column block is a real bin (not padding)
-  static constexpr int kNb = 1 << LG;
+  static constexpr int kGroup = 32 / S;
 
   __device__ __forceinline__ static float plog2p(float p) { return p > 0.f ? p * __log2f(p) : 0.f; }
 
+  // Sum of v over the S lanes from this one on (the first lane of a variable's).
+  __device__ __forceinline__ static float lane_sum(float v) {
+    float w = v, sum = 0.f;  // w: the sum of the next 2^b lanes
+    int off = 0;
+#pragma unroll
+    for (int b = 0; (1 << b) <= S; b++) {
+      if (S & (1 << b)) {
+        sum += off ? __shfl_down_sync(0xffffffffu, w, off) : w;
+        off += 1 << b;
+      }
+      if ((2 << b) <= S) w += __shfl_down_sync(0xffffffffu, w, 1 << b);
+    }
+    return sum;
+  }
+
   __device__ void operator()(int64_t r, int64_t c0, const float (&g)[32], EpiCtx &) const {
     const int lane = threadIdx.x & 31;
-    const int64_t x = r >> LG;
     float t[32];
-    // padding bins are zero columns: skipped (the same positions in every lane)
+    // padding rows of the column operand are zero columns: skipped (the same
+    // positions in every lane)
 #pragma unroll
-    for (int j = 0; j < 32; j++) t[j] = (colmask >> j) & 1u ? plog2p(g[j] * pscale) : 0.f;
-    // segmented sums: t[j] of the first column of each column variable ends
-    // up holding the sum over that variable's bins
+    for (int j = 0; j < kGroup * S; j++)
+      t[j] = (colmask >> j) & 1u ? plog2p(g[j] * pscale) : 0.f;
+    // t[q S]: the sum over column variable q's bins, then over the row variable's
 #pragma unroll
-    for (int l = 0; l < LG; l++) {
+    for (int o = 1; o < S; o *= 2) {
 #pragma unroll
-      for (int j = 0; j < 32; j += 2 << l) t[j] += t[j + (1 << l)];
+      for (int q = 0; q < kGroup; q++)
+#pragma unroll
+        for (int j = 0; j + o < S; j += 2 * o) t[q * S + j] += t[q * S + j + o];
     }
-    // ... and over the row variable's bins (its kNb consecutive lanes)
 #pragma unroll
-    for (int o = kNb >> 1; o > 0; o >>= 1) {
-#pragma unroll
-      for (int j = 0; j < 32; j += kNb) t[j] += __shfl_xor_sync(0xffffffffu, t[j], o);
-    }
-    if ((lane & (kNb - 1)) != 0 || x >= nx) return;
+    for (int q = 0; q < kGroup; q++) t[q * S] = lane_sum(t[q * S]);
+    const int64_t x = (r >> 5) * kGroup + lane / S;
+    if (lane % S != 0 || lane / S >= kGroup || x >= nx) return;
     const float hxx = hx[x];
 #pragma unroll
-    for (int j = 0; j < 32; j += kNb) {
-      const int64_t y = (c0 + j) >> LG;
+    for (int q = 0; q < kGroup; q++) {
+      const int64_t y = (c0 >> 5) * kGroup + q;
       if (y >= ny || (symmetric && y < x)) continue;
-      const float mi = t[j] + hxx + hy[y];
+      const float mi = t[q * S] + hxx + hy[y];
       out[y * ldo + x] = mi;
       if (symmetric && y != x) out[x * ldo + y] = mi;
     }
@@ -1373,33 +1387,38 @@ int tc_plane_map(CUtensorMap *map, const void *base, int64_t rows, int64_t kpad,
   return make_plane_map(map, base, rows, kpad, nplanes, box_rows, bk, f16);
 }
 
-// Mutual information from f16x3 weight planes (rows = variable * 2^lg + bin,
-// each weight times 2^14): the chunked Gram with MiFinish.
+// Mutual information from f16x3 weight planes (mi_stride rows per variable,
+// 32 / stride variables per 32 rows, each weight times 2^14): the chunked Gram
+// with MiFinish.
 int mi_tc(const void *planesX, int64_t rowsX, const void *planesY, int64_t rowsY, int64_t kpad,
-          int lg, int nbins, int64_t nx, int64_t ny, int64_t nsamples, const float *hx,
-          const float *hy, float *out, int symmetric, cudaStream_t s) {
+          int nbins, int64_t nx, int64_t ny, int64_t nsamples, const float *hx, const float *hy,
+          float *out, int symmetric, cudaStream_t s) {
   if (rowsX == 0 || rowsY == 0) return GT_OK;
+  const int stride = mi_stride(nbins);
   unsigned colmask = 0u;
-  for (int j = 0; j < 32; j++)
-    if ((j & ((1 << lg) - 1)) < nbins) colmask |= 1u << j;
+  for (int j = 0; j < 32 / stride * stride; j++)
+    if (j % stride < nbins) colmask |= 1u << j;
   const float pscale = float(1.0 / (268435456.0 * double(nsamples)));
   // FP32 chunks of 512 samples: 15 % faster than 256 at 10 bins x 1000 samples, with a
   // largest MI error of 7.5e-6 bits against the FP64 oracle (4.1e-6 with 256)
-  auto run = [&](auto lgc) {
-    constexpr int LG = decltype(lgc)::value;
-    MiFinish<LG> fin{out, hx, hy, nx, ny, nx, pscale, symmetric, colmask};
+  auto run = [&](auto st) {
+    constexpr int S = decltype(st)::value;
+    MiFinish<S> fin{out, hx, hy, nx, ny, nx, pscale, symmetric, colmask};
     return launch_gram<tc::KIND_F16X3, 32, true>(planesX, rowsX, planesY, rowsY, kpad,
                                                  symmetric ? kUpper : kFull, 512 / 32, fin,
                                                  "mi_gram", s);
   };
-  switch (lg) {
-    case 0: return run(std::integral_constant<int, 0>{});
+  switch (stride) {
     case 1: return run(std::integral_constant<int, 1>{});
     case 2: return run(std::integral_constant<int, 2>{});
-    case 3: return run(std::integral_constant<int, 3>{});
     case 4: return run(std::integral_constant<int, 4>{});
     case 5: return run(std::integral_constant<int, 5>{});
-    default: return fail(GT_EINVAL, "bins beyond the tensor-core path (%d)", 1 << lg);
+    case 6: return run(std::integral_constant<int, 6>{});
+    case 8: return run(std::integral_constant<int, 8>{});
+    case 10: return run(std::integral_constant<int, 10>{});
+    case 16: return run(std::integral_constant<int, 16>{});
+    case 32: return run(std::integral_constant<int, 32>{});
+    default: return fail(GT_EINVAL, "bins beyond the tensor-core path (%d)", nbins);
   }
 }
 

@@ -84,12 +84,20 @@ int pearson_exact_band(const void *zA, int64_t nA, const void *zB, int64_t nB, i
 int pearson_pairwise_tc(const float *dA, int64_t nA, const float *dB, int64_t nB, int64_t n,
                         const PearsonOut &out, const int *run_if, cudaStream_t s);
 
+// Rows of the mutual-information operand per variable: the fewest such that
+// 32 / stride whole variables fill a group of 32 rows (9 or 10 bins: 3 variables of
+// 10 rows, where powers of two would hold 2 of 16).  Three bins keep 4 rows: 10
+// variables of 3 rows are 10 % slower (500 samples x 1000 variables 57 -> 63 us),
+// their sums over lanes costing more than the padding.
+inline int mi_stride(int nbins) { return nbins == 3 ? 4 : 32 / (32 / nbins); }
+
 // gram_tc.cu: B-spline mutual information from f16x3 weight planes ([part]
-// [variable * 2^lg + bin][kpad], weights times 2^14, zero padded), entropies
-// hx, hy; out[y * nx + x] (symmetric: X == Y, both triangles written).
+// [row][kpad], weights times 2^14, zero padded; bin a of variable v is row
+// v / g * 32 + v % g * stride + a with stride = mi_stride(nbins), g = 32 / stride),
+// entropies hx, hy; out[y * nx + x] (symmetric: X == Y, both triangles written).
 int mi_tc(const void *planesX, int64_t rowsX, const void *planesY, int64_t rowsY, int64_t kpad,
-          int lg, int nbins, int64_t nx, int64_t ny, int64_t nsamples, const float *hx,
-          const float *hy, float *out, int symmetric, cudaStream_t s);
+          int nbins, int64_t nx, int64_t ny, int64_t nsamples, const float *hx, const float *hy,
+          float *out, int symmetric, cudaStream_t s);
 
 // C[r][c] = sum_k A_r[k] B_c[k] on tcgen05 from `nsplit` (2 or 3) split-bf16
 // planes ([part][row][kpad], kpad a multiple of 64), stored as row-major float.
