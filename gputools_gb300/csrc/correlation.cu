@@ -7,7 +7,7 @@
 // host (hostSignif, src/correlation.cpp:51-64).
 //
 // Here:
-//  * a prologue computes each variable's mean and norm once, in FP64
+//  * a prologue computes each variable's mean and norm once, as float pairs
 //    (corrected two-pass), and writes the normalised column
 //    z = (x - mean) / ||x - mean||, so r(x, y) = <z_x, z_y>;
 //  * "everything": the Gram contraction runs on tcgen05 tensor cores

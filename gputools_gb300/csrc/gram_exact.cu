@@ -295,15 +295,14 @@ __device__ __forceinline__ void exact_digits(float vh, float vl, uint16_t (&p)[3
 }
 
 // (x - mean) * inv_norm * 2^11 as a float pair (about 2^-46 relative), from
-// the FP64 statistics held as float pairs.
+// the statistics, themselves float pairs.
 struct PairCenterer {
   float mhi, mlo, ihi, ilo;
   __device__ __forceinline__ explicit PairCenterer(const ColStats &s) {
-    mhi = float(s.mean);
-    mlo = float(s.mean - double(mhi));
-    const double inv = s.inv_norm * 2048.0;
-    ihi = float(inv);
-    ilo = float(inv - double(ihi));
+    mhi = s.mhi;
+    mlo = s.mlo;
+    ihi = s.ihi * 2048.f;
+    ilo = s.ilo * 2048.f;
   }
   __device__ __forceinline__ void operator()(float x, float &vh, float &vl) const {
     // x - mhi exactly (TwoSum), then - mlo into the low part

@@ -35,9 +35,10 @@ int tc_map_3d(CUtensorMap *map, CUtensorMapDataType type, const void *base,
 
 // Per-variable statistics of the Pearson prologue.
 struct ColStats {
-  double mean;
-  double inv_norm;  // 1 / sqrt(sum (x - mean)^2), or 0 for a constant variable
-  int flags;        // bit 0: contains NaN; bit 1: zero variance
+  float mhi, mlo;  // mean, as a float pair (about 2^-46 relative)
+  float ihi, ilo;  // 1 / sqrt(sum (x - mean)^2) likewise, or 0 for a constant variable
+  int flags;       // bit 0: contains NaN; bit 1: zero variance
+  int unused;
 };
 
 int launch_colstats(const float *dX, int64_t nvar, int64_t n, int use, ColStats *st,

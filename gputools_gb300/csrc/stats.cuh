@@ -2,8 +2,11 @@
 //
 // GB300's FP64 pipe runs at a small fraction of its FP32 pipe, so the sums
 // over observations are compensated float pairs (Knuth's TwoSum, squares with
-// their exact FMA residual), about 2^-44 relative, and FP64 enters only in
-// the few per-variable operations that finish the statistics.
+// their exact FMA residual), about 2^-44 relative, and so are the few
+// operations that finish a variable's statistics: every lane of its warp makes
+// them, and the 60 or so that they took in FP64 (16 cycles of the SM's FP64 pipe
+// each) were most of the batched prologue (300 problems, 220000 variables:
+// 683 us, now 450).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -22,7 +25,6 @@ struct FloatPairSum {
     lo += (hi - (t - bp)) + (v - bp);
     hi = t;
   }
-  __device__ __forceinline__ double value() const { return double(hi) + double(lo); }
 };
 
 // Sum of the lanes' (hi, lo) pairs, left in every lane.  TwoSum is exact in
@@ -54,17 +56,11 @@ __device__ __forceinline__ void warp_for_each(const float *__restrict__ x, int64
   for (int64_t k = 4 * n4 + lane; k < n; k += 32) f(x[k]);
 }
 
-// 1/N in double from a float reciprocal and one Newton step.
-__device__ __forceinline__ double recip_d(double N) {
-  const double y = double(1.f / float(N));
-  return y * (2.0 - N * y);
-}
-
 // Sum of x[0..n) as a float pair in every lane, with the count of non-NaN
 // values, of NaN values, and the largest finite magnitude; values are
 // multiplied by the power of two `sc` first.
 struct WarpSums {
-  double S;
+  float hi, lo;
   int cnt, nan;
   float amax;
 };
@@ -83,10 +79,10 @@ __device__ __forceinline__ WarpSums warp_sums(const float *__restrict__ x, int64
       if (a <= 3.4e38f) amax = fmaxf(amax, a);
     }
   });
-  float hi = s.hi, lo = s.lo;
-  warp_pair_sum(hi, lo);
   WarpSums r;
-  r.S = double(hi) + double(lo);
+  r.hi = s.hi;
+  r.lo = s.lo;
+  warp_pair_sum(r.hi, r.lo);
   r.cnt = __reduce_add_sync(FULL, cnt);
   r.nan = __reduce_add_sync(FULL, nan);
   r.amax = __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(amax)));
@@ -111,19 +107,22 @@ __device__ __forceinline__ ColStats colstats_warp(const float *__restrict__ x, i
   if (w.amax > 0.f) e = int((__float_as_uint(w.amax) >> 23) & 255u) - 127;
   e = e < -126 ? -126 : (e > 126 ? 126 : e);
   const float sc = __uint_as_float(uint32_t(127 - e) << 23);
-  const double dsc = double(sc);
-  double S;
-  if (w.S - w.S == 0.0 || w.amax == 0.f) {
-    S = w.S * dsc;
-  } else {
-    S = warp_sums(x, n, sc).S;  // the plain sum overflowed
+  const float t = w.hi + w.lo;
+  float shi = w.hi * sc, slo = w.lo * sc;
+  if (!(t - t == 0.f) && w.amax != 0.f) {  // the plain sum overflowed
+    const WarpSums ws = warp_sums(x, n, sc);
+    shi = ws.hi;
+    slo = ws.lo;
   }
   const int cnt = w.cnt;
-  const double N = double(cnt);
-  const double invN = cnt > 0 ? recip_d(N) : 0.0;
-  double mean = S * invN;                     // scaled mean
-  mean = fma(fma(-mean, N, S), invN, mean);   // quotient correction
-  const float mhi = float(mean), mlo = float(mean - double(mhi));
+  // the scaled mean as a pair: a quotient, corrected by its residual, then the
+  // residual of the corrected one (exactly 0 for a constant variable)
+  const float N = float(cnt), dN = float(cnt - int(N));  // dN: from 2^24 on
+  const float invN = cnt > 0 ? 1.f / N : 0.f;
+  auto residual = [&](float m) { return fmaf(-m, N, shi) + fmaf(-m, dN, slo); };
+  const float m0 = shi * invN;
+  float mhi = fmaf(residual(m0), invN, m0);
+  float mlo = residual(mhi) * invN;
   FloatPairSum c, ss;
   float sse = 0.f;
   warp_for_each(x, n, [&](float v) {
@@ -137,33 +136,39 @@ __device__ __forceinline__ ColStats colstats_warp(const float *__restrict__ x, i
   float chi = c.hi, clo = c.lo, qhi = ss.hi, qlo = ss.lo + sse;
   warp_pair_sum(chi, clo);
   warp_pair_sum(qhi, qlo);
-  const double C = double(chi) + double(clo);
-  double SS = double(qhi) + double(qlo);
-  if (cnt > 0) {
-    mean += C * invN;
-    SS -= C * (C * invN);
-  }
+  const float C = chi + clo, cm = C * invN;
+  mlo += cm;
+  qlo = fmaf(-C, cm, qlo);
+  const float m = mhi + mlo, q = qhi + qlo;
+  mlo -= m - mhi;
+  qlo -= q - qhi;
+  const float up = __uint_as_float(uint32_t(127 + e) << 23);
   ColStats st;
-  st.mean = mean / dsc;  // exact: a power of two
+  st.mhi = m * up;
+  st.mlo = mlo * up;
   st.flags = 0;
   if (use == 0 && w.nan > 0) st.flags |= 1;
-  if (!(SS > 0.0) || cnt < 2) st.flags |= 2;
+  if (!(q > 0.f) || cnt < 2) st.flags |= 2;
   if (st.flags & 2) {
-    st.inv_norm = 0.0;
+    st.ihi = st.ilo = 0.f;
   } else {
-    // 1/sqrt(SS): float estimate, one Newton step in double, then the scale
-    const double y = double(rsqrtf(float(SS)));
-    st.inv_norm = y * (1.5 - 0.5 * SS * y * y) * dsc;
+    // 1/sqrt(q + qlo): an estimate y, then y (1 - r)^(-1/2) with r = 1 - (q + qlo) y^2
+    const float y = rsqrtf(q), y2 = y * y, y2l = fmaf(y, y, -y2);
+    const float r = fmaf(-qlo, y2, fmaf(-q, y2l, fmaf(-q, y2, 1.f)));
+    const float d = y * r * fmaf(0.375f, r, 0.5f);
+    const float inv = y + d;
+    st.ihi = inv * sc;
+    st.ilo = (d - (inv - y)) * sc;
   }
   return st;
 }
 
 // z = (x - mean) * inv_norm in float arithmetic with the mean as a float
-// pair: the float rounding of the FP64 value to within a couple of ulp.
+// pair: the float rounding of the exact value to within a couple of ulp.
 struct Centerer {
   float mhi, mlo, inv;
   __device__ __forceinline__ explicit Centerer(const ColStats &s)
-      : mhi(float(s.mean)), mlo(float(s.mean - double(float(s.mean)))), inv(float(s.inv_norm)) {}
+      : mhi(s.mhi), mlo(s.mlo), inv(s.ihi) {}
   __device__ __forceinline__ float operator()(float x) const { return ((x - mhi) - mlo) * inv; }
 };
 

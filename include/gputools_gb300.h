@@ -268,7 +268,7 @@ int gt_hclust_format(int len, const int *sub, const int *sup, int *merge, int *o
 /* dL/dX of C = cor(X) (Pearson, "everything") given G = dL/dC.
  * X variable-major p x n (X[j*n + k]), G row-major p x p (G[i*p + j] =
  * dL/dC_ij; G and its transpose give the same result), dX like X.  Means and
- * norms are recomputed in FP64; the contraction W = (G + G^T) Z runs on the
+ * norms are recomputed as float pairs; the contraction W = (G + G^T) Z runs on the
  * selected Gram path.  Constant variables get a zero gradient. */
 int gt_cor_backward_device(const float *d_X, int64_t p, int64_t n,
                            const float *d_G, float *d_dX, void *stream);
