@@ -252,6 +252,9 @@ int pearson_impl(int use, const float *dA, int64_t nA, const float *dB, int64_t 
     GT_TRY(any_nan_flag(dA, nA * n, symmetric ? nullptr : dB, nB * n, &nan_flag, s));
     po.gate = nan_flag;
   }
+  if (use == GT_EVERYTHING && path == GT_GRAM_TC_F16X3 && n > 0 &&
+      pearson_fma_wins(nA, nB, n, symmetric))
+    return pearson_fma(dA, nA, dB, nB, n, po, s);
   if (tc) {
     void *zA = nullptr, *zB = nullptr;
     int64_t kpad = 0;

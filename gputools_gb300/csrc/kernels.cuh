@@ -60,6 +60,11 @@ struct PearsonOut {
 int pearson_tc(const void *d_zA, int64_t nA, const void *d_zB, int64_t nB, int64_t kpad,
                int kind, const PearsonOut &out, cudaStream_t st);
 
+// pearson_fma.cu: small "everything" problems on CUDA cores, statistics included.
+bool pearson_fma_wins(int64_t nA, int64_t nB, int64_t n, int symmetric);
+int pearson_fma(const float *dA, int64_t nA, const float *dB, int64_t nB, int64_t n,
+                const PearsonOut &out, cudaStream_t s);
+
 // gram_exact.cu: the error-free Pearson Gram (GT_GRAM_TC_F16X6): the
 // prologue writes three fixed-point fp16 digit planes per variable
 // ([plane][variable][kpad], kpad a multiple of 64), the Gram sums their

@@ -62,7 +62,9 @@ enum gt_gram_path {
   GT_GRAM_TC_BF16X3 = 0, /* tcgen05, each operand split hi+lo bf16, 3 products */
   GT_GRAM_TC_BF16X6 = 1, /* tcgen05, 3-way bf16 split, 6 products             */
   GT_GRAM_FP32 = 2,      /* plain FP32 CUDA-core path                         */
-  GT_GRAM_TC_F16X3 = 3,  /* tcgen05, power-of-two scaled hi+lo fp16, 3 products */
+  GT_GRAM_TC_F16X3 = 3,  /* tcgen05, power-of-two scaled hi+lo fp16, 3 products;
+                            Pearson problems too small to fill the chip with its
+                            tiles run as FP32 multiply-adds, with a smaller error */
   GT_GRAM_TC_F16X6 = 4   /* tcgen05, three fixed-point fp16 digits per value whose
                             products sum exactly in FP32 (error-free split),
                             6 products; Pearson only (gpuDist runs f16x3) */
