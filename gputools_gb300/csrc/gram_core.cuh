@@ -161,6 +161,63 @@ inline TileSpace make_tiles(int64_t nr, int64_t nc, int mode, int64_t group) {
   return ts;
 }
 
+// The 256 x 256 tiles of a CTA pair (each CTA the 128 rows of its rank): all of
+// them, or (symmetric) those with row block <= column block, in the same bands
+// of `1 << group_log2` column blocks, row block by row block.
+struct PairSpace {
+  int64_t tr, tc, ntiles;  // row blocks, column blocks, tiles (below 2^31)
+  int group_log2;
+  int symmetric;
+};
+
+__host__ __device__ inline void pair_coords(const PairSpace &ps, int64_t t64, int64_t &ti,
+                                            int64_t &tj) {
+  const uint32_t t = uint32_t(t64), tr = uint32_t(ps.tr), tc = uint32_t(ps.tc);
+  const uint32_t lg = uint32_t(ps.group_log2), G = 1u << lg;
+  uint32_t c0, u, full;  // the band's first column, the tile's place in it, its full rows
+  if (ps.symmetric) {
+    int32_t j = int32_t((sqrtf(float(t) * 8.f + 1.f) - 1.f) * 0.5f);  // t's column, in
+    if (j < 0) j = 0;                                                 // column-major order
+    while (uint64_t(j + 1) * uint64_t(j + 2) / 2 <= t) j++;
+    while (uint64_t(j) * uint64_t(j + 1) / 2 > t) j--;
+    c0 = (uint32_t(j) >> lg) << lg;
+    u = t - uint32_t(uint64_t(c0) * uint64_t(c0 + 1) / 2);
+    full = c0 + 1;  // rows 0 .. c0 meet every column of the band
+  } else {
+    c0 = (t / (tr << lg)) << lg;
+    u = t - c0 * tr;
+    full = tr;
+  }
+  const uint32_t g = tc - c0 < G ? tc - c0 : G;
+  if (u < full * g) {
+    const uint32_t i = u / g;
+    ti = i;
+    tj = c0 + (u - i * g);
+    return;
+  }
+  u -= full * g;
+  for (uint32_t w = 1;; w++) {  // row c0 + w meets the last g - w columns
+    const uint32_t cnt = g - w;
+    if (u < cnt) {
+      ti = c0 + w;
+      tj = c0 + w + u;
+      return;
+    }
+    u -= cnt;
+  }
+}
+
+inline PairSpace make_pair_space(int64_t nr, int64_t nc, int symmetric, int64_t group) {
+  PairSpace ps;
+  ps.tr = cdiv(nr, 2 * kBM);
+  ps.tc = cdiv(nc, kBN);
+  ps.symmetric = symmetric;
+  ps.ntiles = symmetric ? ps.tc * (ps.tc + 1) / 2 : ps.tr * ps.tc;
+  ps.group_log2 = 0;
+  while ((int64_t(2) << ps.group_log2) <= group) ps.group_log2++;
+  return ps;
+}
+
 // Band width for operand planes of `panel_bytes` per 256-row B panel: as
 // many B panels as fit in about 48 MB of L2, at most 16 (make_tiles rounds
 // it down to a power of two).  Measured at 20000 x 4096: the error-free Gram
@@ -374,6 +431,40 @@ struct SingleWork {
   }
 };
 
+// One problem in 256 x 256 tiles dealt round-robin to CTA pairs (clusters of
+// two): row0 is the pair's first row.
+template <class Fin>
+struct PairWork {
+  CUtensorMap ma, mb;
+  PairSpace ps;
+  int64_t nk;
+  Fin fin;
+  __device__ bool tile(int64_t cursor, TileRef &ref) const {
+    const int64_t t = int64_t(blockIdx.x >> 1) + cursor * int64_t(gridDim.x >> 1);
+    if (t >= ps.ntiles) return false;
+    int64_t ti, tj;
+    pair_coords(ps, t, ti, tj);
+    ref.row0 = ti * (2 * kBM);
+    ref.col0 = tj * kBN;
+    ref.ma = &ma;
+    ref.mb = &mb;
+    ref.nk = nk;
+    ref.prob = 0;
+    return true;
+  }
+  static constexpr bool kPrefetch = false;
+  __device__ bool skip() const {
+    if constexpr (std::is_same<Fin, PearsonFinish>::value) return fin.skip();
+    return false;
+  }
+  __device__ const Fin &finish(const TileRef &) const { return fin; }
+  __device__ void drain(EpiCtx &ctx) const { fin.drain(ctx); }
+  __device__ void prefetch() const {
+    tc::prefetch_tensormap(&ma);
+    tc::prefetch_tensormap(&mb);
+  }
+};
+
 // One problem whose tiles come from a table of (row0, col0) built on the host
 // (a band of rows at a time, in the order the table lists them); the cursor
 // looks each entry up a tile ahead.
@@ -429,6 +520,32 @@ inline void band_tiles(int64_t nr, int64_t nc, bool symmetric, int64_t band_bloc
           tiles.push_back(make_int2(int(ti * kBM), int(tj * kBN)));
     offsets.push_back(int64_t(tiles.size()));
   }
+}
+
+// Launches a persistent kernel of CTA pairs (clusters of two CTAs) over `ntiles`
+// tiles: as many pairs as the device holds at once, at most one per tile.
+template <class Kern, class... Args>
+int launch_pairs(Kern kern, int64_t ntiles, int threads, int smem, cudaStream_t s,
+                 const Args &...args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 2;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cfg.blockDim = dim3(unsigned(threads));
+  cfg.dynamicSmemBytes = size_t(smem);
+  cfg.stream = s;
+  cfg.gridDim = dim3(unsigned(sm_count() / 2 * 2));
+  int pairs = 0;
+  GT_CUDA(cudaOccupancyMaxActiveClusters(&pairs, kern, &cfg));
+  if (pairs < 1) return fail(GT_ECUDA, "no room for a pair of CTAs");
+  cfg.gridDim = dim3(unsigned(2 * (ntiles < pairs ? ntiles : int64_t(pairs))));
+  GT_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
+  count_launch();
+  return GT_OK;
 }
 
 __device__ __forceinline__ int64_t find_segment(const int64_t *__restrict__ prefix, int64_t n,

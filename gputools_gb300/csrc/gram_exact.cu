@@ -32,13 +32,20 @@
 //
 // Kernel.  Persistent, one CTA per SM, 10 warps, on the 128 x 256 tiles of
 // the other Gram kernels, each processed as two 128 x 128 halves (a half that
-// lies wholly below the diagonal of a symmetric problem is skipped):
+// lies wholly below the diagonal of a symmetric problem is skipped).  Problems
+// that fill the chip with 256 x 256 tiles run them on pairs of CTAs
+// (cta_group::2, clusters of two): the halves are 256 x 128, each CTA holding 128
+// rows of A and 64 of B, so a stage fetches a quarter less.  What bounds both
+// is the power limit: with the operands left in place (no copies at all) the
+// MMAs alone take 6.0 ms of the 6.4 that the pairs take at 20000 x 4096 (1.53
+// PFLOP/s; cuBLAS holds 1.71 under the cap), 6.7 before pairs and 128-byte rows.
 //   warp 0      TMA producer: 3-D loads of the three digit planes of the A
-//               (128-row) and B (128-row) boxes, 32 k per stage;
+//               (128-row) and B (128- or 64-row) boxes, 64 k per stage;
 //   warp 1      allocates 512 TMEM columns (three 128 x 128 accumulators) and
 //               one thread issues six tcgen05.mma (M = 128, N = 128, K = 16)
 //               per k-step: P0.P0 -> S0, P0.X1, X1.P0 -> S1,
-//               P0.X2, X2.P0, X1.X1 -> S2;
+//               P0.X2, X2.P0, X1.X1 -> S2 (of a pair: the even CTA's thread,
+//               M = 256, and both CTAs' copies count on its barriers);
 //   warps 2..9  epilogue: two warps per TMEM lane quarter, 64 columns each;
 //               they read the three sums, release the accumulators, then run
 //               the Pearson finish while the next half's MMAs run.
@@ -57,19 +64,26 @@ namespace gt {
 namespace {
 
 constexpr int kXB = 128;     // columns of a half tile (MMA N)
-constexpr int kXBK = 32;     // k per stage (64-byte rows, 64-byte swizzle)
+// k per stage: 128-byte rows with the 128-byte swizzle.  Two stages of 64 take
+// 6.91 ms at 20000 x 4096 where five of 32 take 7.21 (pairs; 7.07 and 7.35 single):
+// half as many rows to fetch.
+constexpr int kXBK = 64;
 constexpr int kXPlanes = 3;  // digit planes P0, X1, X2
 constexpr int kXEpi = 8;     // epilogue warps
 constexpr int kXThreads = 64 + 32 * kXEpi;
 constexpr int kXCols = 4 * kXB / kXEpi;  // columns per epilogue warp (64)
 constexpr int kXATile = kBM * kXBK * 2;  // 8 KB
-constexpr int kXBTile = kXB * kXBK * 2;  // 8 KB
-constexpr int kXStage = kXPlanes * (kXATile + kXBTile);
 constexpr int kXEpiBytes = kXEpi * kEpiTileFloats * 4;
-constexpr int kXStagesRaw = (kMaxSmem - 1024 - 256 - kXEpiBytes) / kXStage;
-constexpr int kXStages = kXStagesRaw > 6 ? 6 : kXStagesRaw;
-constexpr int kXSmem = kXStages * kXStage + 1024 + 256 + kXEpiBytes;
-static_assert(kXStages >= 3, "the exact Gram needs at least three stages");
+template <bool PAIR>
+struct ExactCfg {
+  static constexpr int BROWS = PAIR ? kXB / 2 : kXB;  // B rows that this CTA loads
+  static constexpr int BTILE = BROWS * kXBK * 2;
+  static constexpr int STAGE = kXPlanes * (kXATile + BTILE);
+  static constexpr int RAW = (kMaxSmem - 1024 - 256 - kXEpiBytes) / STAGE;
+  static constexpr int STAGES = RAW > 6 ? 6 : RAW;
+  static constexpr int SMEM = STAGES * STAGE + 1024 + 256 + kXEpiBytes;
+  static_assert(STAGES >= 2, "the exact Gram needs at least two stages");
+};
 static_assert(kXCols == 64, "two 32-column blocks per epilogue warp");
 
 // Products of a k-step: (A plane, B plane, accumulator).
@@ -89,9 +103,11 @@ __device__ __forceinline__ bool half_live(const PearsonFinish &fin, const TileRe
   return true;
 }
 
-template <class Work>
+template <class Work, bool PAIR>
 __global__ void __launch_bounds__(kXThreads, 1)
 gram_exact_kernel(const __grid_constant__ Work work, const tc::WaitCfg wc) {
+  using C = ExactCfg<PAIR>;
+  constexpr int kXStages = C::STAGES, kXStage = C::STAGE, kXBTile = C::BTILE;
   if (work.skip()) return;  // a gated launch whose gate is closed: before any setup
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
@@ -106,21 +122,23 @@ gram_exact_kernel(const __grid_constant__ Work work, const tc::WaitCfg wc) {
   float *epi_smem = reinterpret_cast<float *>(smem + kXStages * kXStage + 256);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = PAIR ? int(tc::cluster_rank()) : 0;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kXStages; s++) {
       tc::mbar_init(&full[s], 1);
       tc::mbar_init(&empty[s], 1);
     }
     tc::mbar_init(accf, 1);
-    tc::mbar_init(acce, kXEpi);
+    tc::mbar_init(acce, PAIR ? 2 * kXEpi : kXEpi);
     tc::mbar_init(mma_done, 1);
     *abort_flag = 0;
     tc::fence_barrier_init();
   }
   if (warp == 0 && lane == 0) work.prefetch();
-  if (warp == 1) tc::tmem_alloc(tmem_slot, 4 * kXB);
+  if (warp == 1) tc::tmem_alloc<PAIR>(tmem_slot, 4 * kXB);
   tc::tc_fence_before();
   __syncthreads();
+  if constexpr (PAIR) tc::cluster_sync();  // both CTAs' barriers and TMEM are there
   tc::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
@@ -135,7 +153,8 @@ gram_exact_kernel(const __grid_constant__ Work work, const tc::WaitCfg wc) {
         const auto &fin = work.finish(ref);
         for (int h = 0; h < 2 && go; h++) {
           if (!half_live(fin, ref, h)) continue;
-          const int32_t c0 = int32_t(ref.col0 + int64_t(h) * kXB);
+          const int32_t r0 = int32_t(ref.row0) + rank * kBM;
+          const int32_t c0 = int32_t(ref.col0 + int64_t(h) * kXB) + rank * C::BROWS;
           for (int64_t kb = 0; kb < ref.nk; kb++, it++) {
             const int s = int(it % kXStages);
             const uint32_t use = uint32_t(it / kXStages);
@@ -145,20 +164,25 @@ gram_exact_kernel(const __grid_constant__ Work work, const tc::WaitCfg wc) {
               break;
             }
             uint8_t *st = smem + s * kXStage;
-            tc::mbar_arrive_expect_tx(&full[s], kXStage);
+            // a pair's copies all count on the even CTA's barrier
+            if (rank == 0) tc::mbar_arrive_expect_tx(&full[s], (PAIR ? 2 : 1) * kXStage);
+            auto load = [&](void *dst, const CUtensorMap *map, int32_t row, int p) {
+              if constexpr (PAIR)
+                tc::tma_load_3d_pair(dst, map, &full[s], int32_t(kb * kXBK), row, p);
+              else
+                tc::tma_load_3d(dst, map, &full[s], int32_t(kb * kXBK), row, p);
+            };
+#pragma unroll
+            for (int p = 0; p < kXPlanes; p++) load(st + p * kXATile, ref.ma, r0, p);
 #pragma unroll
             for (int p = 0; p < kXPlanes; p++)
-              tc::tma_load_3d(st + p * kXATile, ref.ma, &full[s], int32_t(kb * kXBK),
-                              int32_t(ref.row0), p);
-#pragma unroll
-            for (int p = 0; p < kXPlanes; p++)
-              tc::tma_load_3d(st + kXPlanes * kXATile + p * kXBTile, ref.mb, &full[s],
-                              int32_t(kb * kXBK), c0, p);
+              load(st + kXPlanes * kXATile + p * kXBTile, ref.mb, c0, p);
           }
         }
       }
       // drain: no bulk copy may still be writing shared memory at exit
-      if (*abort_flag) {
+      // (a pair that gives up lets time pass below instead)
+      if (!PAIR && *abort_flag) {
         for (int s = 0; s < kXStages; s++) {
           const int64_t fills = it / kXStages + (s < it % kXStages ? 1 : 0);
           if (fills > 0) tc::mbar_wait_bounded(&full[s], uint32_t((fills - 1) & 1), kDrainLimitNs);
@@ -169,12 +193,13 @@ gram_exact_kernel(const __grid_constant__ Work work, const tc::WaitCfg wc) {
   } else if (warp == 1) {
     if (lane == 0) {
       // ------------------------------------------------ MMA issuer
-      constexpr uint32_t idesc = tc::idesc_f32acc(kBM, kXB, 0u /* fp16 */);
+      // of a pair: the even CTA's thread
+      constexpr uint32_t idesc = tc::idesc_f32acc(PAIR ? 2 * kBM : kBM, kXB, 0u /* fp16 */);
       int64_t it = 0, hc = 0;
       bool ok = true;
       TileRef ref;
       TileCursor<Work> tiles(work, 0, 1);
-      while (ok && tiles.next(ref)) {
+      while (rank == 0 && ok && tiles.next(ref)) {
         const auto &fin = work.finish(ref);
         for (int h = 0; h < 2 && ok; h++) {
           if (!half_live(fin, ref, h)) continue;
@@ -200,23 +225,32 @@ gram_exact_kernel(const __grid_constant__ Work work, const tc::WaitCfg wc) {
               for (int p = 0; p < 6; p++) {
                 int pa, pb, acc;
                 exact_product(p, pa, pb, acc);
-                const uint64_t ad = tc::smem_desc_kmajor(sa + pa * kXATile + k * 32, 64);
-                const uint64_t bd = tc::smem_desc_kmajor(sb + pb * kXBTile + k * 32, 64);
+                const uint64_t ad = tc::smem_desc_kmajor(sa + pa * kXATile + k * 32, 128);
+                const uint64_t bd = tc::smem_desc_kmajor(sb + pb * kXBTile + k * 32, 128);
                 // the first product into each sum starts it
-                const bool first = kb == 0 && k == 0 && (p == 0 || p == 1 || p == 3);
-                tc::umma_bf16(tmem_base + uint32_t(acc * kXB), ad, bd, idesc, first ? 0u : 1u);
+                const uint32_t more = kb == 0 && k == 0 && (p == 0 || p == 1 || p == 3) ? 0u : 1u;
+                if constexpr (PAIR)
+                  tc::umma_bf16_pair(tmem_base + uint32_t(acc * kXB), ad, bd, idesc, more);
+                else
+                  tc::umma_bf16(tmem_base + uint32_t(acc * kXB), ad, bd, idesc, more);
               }
             }
-            tc::umma_commit(&empty[s]);
+            if constexpr (PAIR) tc::umma_commit_pair(&empty[s]);
+            else tc::umma_commit(&empty[s]);
           }
           if (!ok) break;
-          tc::umma_commit(accf);
+          if constexpr (PAIR) tc::umma_commit_pair(accf);
+          else tc::umma_commit(accf);
           hc++;
         }
       }
       if (!ok) *abort_flag = 1;
       // every MMA issued above has finished before TMEM is released
-      tc::umma_commit(mma_done);
+      if constexpr (PAIR) {
+        if (rank == 0) tc::umma_commit_pair(mma_done);
+      } else {
+        tc::umma_commit(mma_done);
+      }
       tc::mbar_wait_bounded(mma_done, 0u, kDrainLimitNs);
     }
     __syncwarp();
@@ -236,7 +270,7 @@ gram_exact_kernel(const __grid_constant__ Work work, const tc::WaitCfg wc) {
       const auto &fin = work.finish(ref);
       for (int h = 0; h < 2; h++) {
         if (!half_live(fin, ref, h)) continue;
-        const int64_t r = ref.row0 + q * 32 + lane;
+        const int64_t r = ref.row0 + rank * kBM + q * 32 + lane;
         const int64_t col = ref.col0 + int64_t(h) * kXB + part * kXCols;
         ctx.rbase = r - lane;
         ctx.col0 = col;
@@ -263,7 +297,10 @@ gram_exact_kernel(const __grid_constant__ Work work, const tc::WaitCfg wc) {
         }
         tc::tc_fence_before();
         __syncwarp();
-        if (lane == 0) tc::mbar_arrive(acce);
+        if (lane == 0) {
+          if constexpr (PAIR) tc::mbar_arrive_cta(acce, 0);
+          else tc::mbar_arrive(acce);
+        }
         hc++;
         fin.begin_tile(r, ctx);
         fin(r, col, g[0], ctx);
@@ -275,9 +312,18 @@ gram_exact_kernel(const __grid_constant__ Work work, const tc::WaitCfg wc) {
   }
   __syncthreads();
   if (*abort_flag && threadIdx.x == 0) atomicOr(wc.err, 1);
+  if constexpr (PAIR) {
+    if (*abort_flag && threadIdx.x == 0) tc::pass_time(tc::kCopyTimeNs);
+    __syncthreads();
+    tc::cluster_sync();  // the even CTA's MMAs use both CTAs' memory and arrive in both
+  }
   if (warp == 1) {
     tc::tc_fence_after();
-    tc::tmem_dealloc(tmem_base, 4 * kXB);
+    tc::tmem_dealloc<PAIR>(tmem_base, 4 * kXB);
+  }
+  if constexpr (PAIR) {
+    __syncwarp();
+    tc::cluster_sync();
   }
 }
 
@@ -396,13 +442,26 @@ int launch_exact(const W &w, int64_t ntiles, cudaStream_t s) {
   if (ntiles == 0) return GT_OK;
   tc::WaitCfg wc;
   GT_TRY(make_wait_cfg(&wc));
-  auto kern = gram_exact_kernel<W>;
-  GT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kXSmem));
+  auto kern = gram_exact_kernel<W, false>;
+  constexpr int smem = ExactCfg<false>::SMEM;
+  GT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   const int64_t grid = ntiles < sm_count() ? ntiles : sm_count();
   ProfScope prof("pearson_gram", s);
-  kern<<<unsigned(grid), kXThreads, kXSmem, s>>>(w, wc);
+  kern<<<unsigned(grid), kXThreads, smem, s>>>(w, wc);
   count_launch();
   GT_CUDA(cudaGetLastError());
+  return GT_OK;
+}
+
+// The pair kernel: persistent clusters of two CTAs.
+int launch_exact_pair(const PairWork<PearsonFinish> &w, cudaStream_t s) {
+  tc::WaitCfg wc;
+  GT_TRY(make_wait_cfg(&wc));
+  auto kern = gram_exact_kernel<PairWork<PearsonFinish>, true>;
+  constexpr int smem = ExactCfg<true>::SMEM;
+  GT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  ProfScope prof("pearson_gram", s);
+  GT_TRY(launch_pairs(kern, w.ps.ntiles, kXThreads, smem, s, w, wc));
   return GT_OK;
 }
 
@@ -436,12 +495,27 @@ int pearson_exact(const void *zA, int64_t nA, const void *zB, int64_t nB, int64_
   if (nA == 0 || nB == 0) return GT_OK;
   if (!out.corr && !out.ts && !out.pairs) return GT_OK;
   if (kpad <= 0 || kpad % kKPad) return fail(GT_EINVAL, "bad padded K (%lld)", (long long)kpad);
+  const int64_t panel = int64_t(kBN) * kpad * 2 * kXPlanes;
+  // pairs: twice as wide bands, measured with 8 / 16 / 32 / 64 panels of 6 MB 6.98 /
+  // 6.82 / 6.88 / 7.04 ms
+  const PairSpace ps = make_pair_space(nA, nB, out.symmetric, band_group(panel / 2));
+  // at least one tile for every pair; below that single CTAs' smaller tiles
+  // spread better
+  if (2 * ps.ntiles >= sm_count() && ps.ntiles <= 2147483647LL && nA > kBM) {
+    PairWork<PearsonFinish> w;
+    GT_TRY(tc_plane_map(&w.ma, zA, nA, kpad, kXPlanes, kBM, kXBK, true));
+    GT_TRY(tc_plane_map(&w.mb, zB, nB, kpad, kXPlanes, ExactCfg<true>::BROWS, kXBK, true));
+    w.ps = ps;
+    w.nk = kpad / kXBK;
+    w.fin = exact_finish(out, nA, nB);
+    return launch_exact_pair(w, s);
+  }
   using W = SingleWork<PearsonFinish>;
   W w;
   GT_TRY(tc_plane_map(&w.ma, zA, nA, kpad, kXPlanes, kBM, kXBK, true));
   GT_TRY(tc_plane_map(&w.mb, zB, nB, kpad, kXPlanes, kXB, kXBK, true));
   const int mode = out.symmetric ? kUpper : kFull;
-  w.ts = make_tiles(nA, nB, mode, band_group(int64_t(kBN) * kpad * 2 * kXPlanes));
+  w.ts = make_tiles(nA, nB, mode, band_group(panel));
   if (w.ts.ntiles > 2147483647LL)
     return fail(GT_EINVAL, "problem too large (%lld tiles)", (long long)w.ts.ntiles);
   w.nk = kpad / kXBK;
