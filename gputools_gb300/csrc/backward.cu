@@ -650,6 +650,341 @@ __global__ void dist_backward_reduce_kernel(const float *__restrict__ X, int64_t
   }
 }
 
+// ---- each unordered pair once
+// The adjoint of the distances in 64 x 64 tiles of point pairs i < j: the
+// distance, 1 / D and W_ij are formed once per unordered pair and used for both
+// points (the kernel above forms them for (i, j) and for (j, i)).
+//   phase 1: thread (ty, tx) takes the pairs of rows ty + 16 a and columns tx +
+//            16 b; the squares sum in the same four chains over k mod 4 as above,
+//            two chains to a packed FP32 operation, so D is the same number;
+//            W goes to shared memory in both orientations;
+//   phase 2: warps 0..3 add sum_j W_ij x_j to the row block's running sums, warps
+//            4..7 form sum_i W_ij x_i of the column block, 4 rows x DMAX / 8
+//            dimensions a thread.
+// A block walks `len` consecutive tiles of the row-major list (I, J >= I).  The
+// column sums of every tile, and the row sums whenever the row block or the
+// segment ends, go to partial buffers that a second kernel adds in a fixed order.
+// Bound by issue and latency at 16 warps an SM (61 % of the issue slots): 185
+// instructions a pair, where the ordered kernel makes 380.  8192 x 32 (MDS stress):
+// 296 us per call, 455 with ordered pairs; the gradient's error 0.8e-7 (1.2e-7).
+constexpr int kPtT = 64, kPtThreads = 256;
+
+template <int DMAX>
+struct PtSmem {
+  static constexpr int LD = DMAX + 4;   // rows 4 banks apart (mod 32)
+  // W rows 8 banks apart, W^T rows 4: a warp's 4 x 8 stores meet no conflicts
+  static constexpr int LW = kPtT + 8, LT = kPtT + 4;
+  static constexpr int X = kPtT * LD, W = kPtT * LW, WT = kPtT * LT;
+  static constexpr int SUMS = kPtT * DMAX;  // the row block's running sums
+  static constexpr int BYTES = (3 * X + W + WT + SUMS) * 4;
+};
+
+// The partial buffers: column sums of tile (I, J) at J (J + 1) / 2 + I, row sums
+// of row block I in segment q at q + I (both lists of [64][dim] blocks, with
+// [64] sums of W beside them).
+struct PtPartials {
+  float *col, *colw, *row, *roww;
+  double *loss;  // one per segment
+};
+
+__host__ __device__ inline int64_t pt_first(int64_t I, int64_t nb) { return I * nb - I * (I - 1) / 2; }
+
+template <int DMAX, int MODE>
+__global__ void __launch_bounds__(kPtThreads, 2)
+dist_pairs_kernel(const float *__restrict__ X, int64_t n, int64_t dim,
+                  const float *__restrict__ aux, int64_t nb, int64_t len, PtPartials out) {
+  using L = PtSmem<DMAX>;
+  constexpr int DPT = DMAX / 8;  // dimensions per thread in phase 2
+  extern __shared__ __align__(16) float dsm[];
+  float *xi = dsm, *xj = dsm + L::X;  // [64][LD]; xj double-buffered
+  float *ws = xj + 2 * L::X, *wt = ws + L::W;  // W_ij at ws[i][j] and wt[j][i]
+  float *rsum = wt + L::WT;                    // [128 threads][4][DPT]
+  __shared__ float wred[2][4][kPtT];           // sums of W: columns; rows (running)
+  __shared__ double lred[kPtThreads / 32];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int ty = 4 * (warp >> 1) + (lane >> 3), tx = 8 * (warp & 1) + (lane & 7);
+  const int side = warp >> 2, w4 = warp & 3;           // phase 2: row or column sums
+  const int rg = lane >> 1, dg = 2 * w4 + (lane & 1);  // ... of rows 4 rg .., dimensions DPT dg ..
+  const bool vec = (dim & 3) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
+
+  auto load = [&](float *dst, int64_t p0) {  // points p0 .. p0 + 63, zero past the end
+    if (vec) {
+      for (int e = tid; e < kPtT * DMAX / 4; e += kPtThreads) {
+        const int r = e / (DMAX / 4), k = 4 * (e - r * (DMAX / 4));
+        const bool ok = p0 + r < n && k < dim;
+        cp_async16(dst + r * L::LD + k, ok ? X + (p0 + r) * dim + k : X, ok ? 16 : 0);
+      }
+    } else {
+      for (int e = tid; e < kPtT * DMAX; e += kPtThreads) {
+        const int r = e / DMAX, k = e - r * DMAX;
+        const bool ok = p0 + r < n && k < dim;
+        cp_async4(dst + r * L::LD + k, ok ? X + (p0 + r) * dim + k : X, ok ? 4 : 0);
+      }
+    }
+    cp_async_commit();
+  };
+
+  // the segment's first tile (I, J)
+  const int64_t total = nb * (nb + 1) / 2, t0 = int64_t(blockIdx.x) * len;
+  const int64_t t1 = t0 + len < total ? t0 + len : total;
+  int64_t I = 0;
+  {
+    int64_t lo = 0, hi = nb;  // largest I with pt_first(I) <= t0
+    while (hi - lo > 1) {
+      const int64_t mid = (lo + hi) / 2;
+      if (pt_first(mid, nb) <= t0) lo = mid;
+      else hi = mid;
+    }
+    I = lo;
+  }
+  int64_t J = I + (t0 - pt_first(I, nb));
+
+  float acc[4][DPT], wsum[4];
+  // acc to block `slot` of a partial list
+  auto flush = [&](float *sums, int64_t slot) {
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+      float *p = sums + (slot * kPtT + 4 * rg + r) * dim + DPT * dg;
+#pragma unroll
+      for (int k = 0; k < DPT; k++)
+        if (DPT * dg + k < dim) p[k] = acc[r][k];
+    }
+  };
+  // The row sums of each tile are formed from zero and then added to the running
+  // ones (in shared memory): shorter chains of roundings.
+  float *own = rsum + (tid & 127);  // element e at own[128 e]
+  auto zero_rows = [&] {
+    if (side == 0) {
+#pragma unroll
+      for (int e = 0; e < 4 * DPT; e++) own[128 * e] = 0.f;
+      if ((lane & 1) == 0)
+#pragma unroll
+        for (int r = 0; r < 4; r++) wred[1][w4][4 * rg + r] = 0.f;
+    }
+  };
+  zero_rows();
+  FloatPairSum lsum;
+  load(xi, I * kPtT);
+  load(xj, J * kPtT);
+  int b = 0;
+  for (int64_t t = t0; t < t1; t++) {
+    cp_async_wait<0>();
+    __syncthreads();  // xi, xj[b] are in; the other xj and W have been read
+    const bool row_ends = J + 1 == nb;
+    const int64_t i0 = I * kPtT, j0 = J * kPtT;
+    if (t + 1 < t1) load(xj + (b ^ 1) * L::X, (row_ends ? I + 1 : J + 1) * kPtT);
+    const float *xb = xj + b * L::X;
+    // ------------------------------------------------ phase 1, two columns at a time
+    auto phase1 = [&](auto inner) {
+      constexpr bool INNER = decltype(inner)::value;  // every pair i < j < n
+#pragma unroll 1
+      for (int h = 0; h < 2; h++) {
+        const int64_t gj0 = j0 + tx + 32 * h;
+        float cf[4][2];
+#pragma unroll
+        for (int a = 0; a < 4; a++) {
+          const int64_t gi = i0 + ty + 16 * a;
+          const float *row = aux + (MODE == 0 ? gi * n : n * gi - gi * (gi + 1) / 2 - gi - 1) + gj0;
+#pragma unroll
+          for (int c = 0; c < 2; c++) {
+            const int64_t gj = gj0 + 16 * c;
+            const bool ok = INNER || (gi < gj && gj < n);
+            cf[a][c] = ok ? row[16 * c] : 0.f;
+            if (MODE == 0 && ok) cf[a][c] += aux[gj * n + gi];
+          }
+        }
+        float2 q0[4][2], q1[4][2];  // chains k mod 4 = 0, 1 and 2, 3
+#pragma unroll
+        for (int a = 0; a < 4; a++)
+#pragma unroll
+          for (int c = 0; c < 2; c++) q0[a][c] = q1[a][c] = make_float2(0.f, 0.f);
+        const float *pi = xi + ty * L::LD, *pj = xb + (tx + 32 * h) * L::LD;
+        const float2 minus = make_float2(-1.f, -1.f);
+#pragma unroll 2  // fully unrolled, its loads are hoisted past the registers
+        for (int k = 0; k < DMAX; k += 4) {
+          float4 u[4], v[2];
+#pragma unroll
+          for (int a = 0; a < 4; a++)
+            u[a] = *reinterpret_cast<const float4 *>(pi + 16 * a * L::LD + k);
+#pragma unroll
+          for (int c = 0; c < 2; c++)
+            v[c] = *reinterpret_cast<const float4 *>(pj + 16 * c * L::LD + k);
+#pragma unroll
+          for (int a = 0; a < 4; a++)
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+              const float2 d0 = __ffma2_rn(make_float2(v[c].x, v[c].y), minus,
+                                           make_float2(u[a].x, u[a].y));
+              const float2 d1 = __ffma2_rn(make_float2(v[c].z, v[c].w), minus,
+                                           make_float2(u[a].z, u[a].w));
+              q0[a][c] = __ffma2_rn(d0, d0, q0[a][c]);
+              q1[a][c] = __ffma2_rn(d1, d1, q1[a][c]);
+            }
+        }
+#pragma unroll
+        for (int a = 0; a < 4; a++)
+#pragma unroll
+          for (int c = 0; c < 2; c++) {
+            const int il = ty + 16 * a, jl = tx + 16 * (2 * h + c);
+            const float d2 = (q0[a][c].x + q0[a][c].y) + (q1[a][c].x + q1[a][c].y);
+            float w = 0.f;
+            if (INNER || (i0 + il < j0 + jl && j0 + jl < n)) {
+              float inv_d = 0.f, d = 0.f;
+              if (d2 >= 1e-30f) {
+                inv_d = tc::rsqrt_approx(d2);
+                d = d2 * inv_d;
+              } else if (d2 > 0.f) {
+                d = sqrtf(d2);
+                inv_d = 1.f / d;
+              }
+              if (MODE == 1) {
+                const float e = d - cf[a][c], q = e * e;
+                lsum.add(q);
+                lsum.lo += fmaf(e, e, -q);
+              }
+              // coincident points add to the stress but not to the gradient
+              if (d2 > 0.f) w = MODE == 0 ? cf[a][c] * inv_d : 2.f * (d - cf[a][c]) * inv_d;
+            }
+            ws[il * L::LW + jl] = w;
+            wt[jl * L::LT + il] = w;
+          }
+      }
+    };
+    if (I < J && j0 + kPtT <= n) phase1(std::true_type{});
+    else phase1(std::false_type{});
+    __syncthreads();
+    // ------------------------------------------------ phase 2
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+      wsum[r] = 0.f;
+#pragma unroll
+      for (int k = 0; k < DPT; k++) acc[r][k] = 0.f;
+    }
+    const float *pw = (side ? ws : wt) + 4 * rg, *px = (side ? xi : xb) + DPT * dg;
+    const int lw = side ? L::LW : L::LT;
+    auto rows16 = [&](int m0, auto sum_w) {
+#pragma unroll 8
+      for (int m = m0; m < m0 + kPtT / 4; m++) {
+        const float4 w = *reinterpret_cast<const float4 *>(pw + m * lw);
+        const float wr[4] = {w.x, w.y, w.z, w.w};
+        __align__(16) float v[DPT];
+#pragma unroll
+        for (int k = 0; k < DPT; k += 2) {  // DPT even: 8-byte reads at least
+          if (DPT % 4 == 0 && k % 4 == 0)
+            *reinterpret_cast<float4 *>(v + k) =
+                *reinterpret_cast<const float4 *>(px + m * L::LD + k);
+          else if (DPT % 4 != 0)
+            *reinterpret_cast<float2 *>(v + k) =
+                *reinterpret_cast<const float2 *>(px + m * L::LD + k);
+        }
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+#pragma unroll
+          for (int k = 0; k < DPT; k++) acc[r][k] = fmaf(wr[r], v[k], acc[r][k]);
+          if constexpr (decltype(sum_w)::value) wsum[r] += wr[r];
+        }
+      }
+    };
+#pragma unroll 1
+    for (int q = 0; q < 4; q++) {  // a quarter of the sums of W in each warp
+      if (q == w4) rows16(16 * q, std::true_type{});
+      else rows16(16 * q, std::false_type{});
+    }
+    const bool flush_row = row_ends || t + 1 == t1;  // uniform
+    if (side == 1) {
+      flush(out.col, J * (J + 1) / 2 + I);
+    } else {
+#pragma unroll
+      for (int r = 0; r < 4; r++)
+#pragma unroll
+        for (int k = 0; k < DPT; k++) {
+          acc[r][k] += own[128 * (r * DPT + k)];
+          own[128 * (r * DPT + k)] = flush_row ? 0.f : acc[r][k];
+        }
+      if (flush_row) flush(out.row, int64_t(blockIdx.x) + I);
+    }
+    // the four warps' shares of the sums of W: the columns', the rows' running ones
+    if ((lane & 1) == 0) {
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        float *p = &wred[side ? 0 : 1][w4][4 * rg + r];
+        *p = side ? wsum[r] : *p + wsum[r];
+      }
+    }
+    __syncthreads();
+    if (tid < 2 * kPtT && (tid < kPtT || flush_row)) {
+      const int sd = tid >> 6, r = tid & 63;  // columns: the first 64 threads, rows: the next
+      const float sum = (wred[sd][0][r] + wred[sd][1][r]) + (wred[sd][2][r] + wred[sd][3][r]);
+      if (sd) {
+        out.roww[(int64_t(blockIdx.x) + I) * kPtT + r] = sum;
+#pragma unroll
+        for (int q = 0; q < 4; q++) wred[1][q][r] = 0.f;
+      } else {
+        out.colw[(J * (J + 1) / 2 + I) * kPtT + r] = sum;
+      }
+    }
+    if (row_ends) {
+      I++;
+      J = I;
+      if (t + 1 < t1) load(xi, I * kPtT);  // (the barrier above: its readers are done)
+    } else {
+      J++;
+    }
+    b ^= 1;
+  }
+  if (MODE == 1) {
+    float lh = lsum.hi, ll = lsum.lo;
+    warp_pair_sum(lh, ll);
+    if (lane == 0) lred[warp] = double(lh) + double(ll);
+    __syncthreads();
+    if (tid == 0) {
+      double s = 0.0;
+      for (int q = 0; q < kPtThreads / 32; q++) s += lred[q];
+      out.loss[blockIdx.x] = s;
+    }
+  }
+}
+
+// dX_i = x_i * sum of W - sum of the partial sums, in a fixed order: the row
+// block's segments, then the tiles above it.  A block takes 8 points: a warp
+// sums each one's W, then a thread each (point, dimension), in four chains.
+constexpr int kPtRedRows = 8;
+__global__ void __launch_bounds__(256)
+dist_pairs_reduce_kernel(const float *__restrict__ X, int64_t n, int64_t dim, int64_t nb,
+                         int64_t len, PtPartials in, float *__restrict__ dX) {
+  __shared__ float w[kPtRedRows];
+  const int64_t i0 = int64_t(blockIdx.x) * kPtRedRows, B = i0 / kPtT, r0 = i0 - B * kPtT;
+  const int64_t q0 = pt_first(B, nb) / len, nq = (pt_first(B + 1, nb) - 1) / len - q0 + 1;
+  const int64_t c0 = B * (B + 1) / 2;
+  {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float s = 0.f;
+    for (int64_t q = lane; q < nq; q += 32) s += in.roww[(q0 + q + B) * kPtT + r0 + warp];
+    for (int64_t q = lane; q <= B; q += 32) s += in.colw[(c0 + q) * kPtT + r0 + warp];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) w[warp] = s;
+  }
+  __syncthreads();
+  const int64_t rows = n - i0 < kPtRedRows ? n - i0 : kPtRedRows, step = kPtT * dim;
+  for (int64_t e = threadIdx.x; e < rows * dim; e += 256) {
+    float a[4] = {0.f, 0.f, 0.f, 0.f};
+    const float *p = in.row + (q0 + B) * step + r0 * dim + e;
+    for (int64_t q = 0; q < nq; q++) a[0] += p[q * step];
+    p = in.col + c0 * step + r0 * dim + e;
+    int64_t q = 0;
+    for (; q + 8 <= B + 1; q += 8) {
+      float v[8];
+#pragma unroll
+      for (int u = 0; u < 8; u++) v[u] = p[(q + u) * step];
+#pragma unroll
+      for (int u = 0; u < 8; u++) a[u & 3] += v[u];
+    }
+    for (; q <= B; q++) a[0] += p[q * step];
+    dX[i0 * dim + e] = fmaf(X[i0 * dim + e], w[e / dim], -((a[0] + a[1]) + (a[2] + a[3])));
+  }
+}
+
 // The partial losses summed by one CTA in a fixed order (thread t takes
 // t, t + 1024, ...; then a butterfly in each warp and across the warps), so
 // the result does not depend on timing.
@@ -899,14 +1234,61 @@ int dist_backward_tc(const float *X, int64_t n, int64_t dim, const float *aux, f
   return GT_OK;
 }
 
+// Bytes of the pair kernel's column sums.
+int64_t dist_pairs_bytes(int64_t n, int64_t dim) {
+  const int64_t nb = cdiv(n, kPtT);
+  return nb * (nb + 1) / 2 * kPtT * (dim + 1) * 4;
+}
+
+template <int DMAX, int MODE>
+int dist_backward_pairs(const float *X, int64_t n, int64_t dim, const float *aux, float *dX,
+                        double *loss, cudaStream_t s) {
+  using L = PtSmem<DMAX>;
+  auto kern = dist_pairs_kernel<DMAX, MODE>;
+  GT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::BYTES));
+  int per = 0;
+  GT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, kPtThreads, L::BYTES));
+  const int64_t slots = int64_t(sm_count()) * (per < 1 ? 1 : per);
+  const int64_t nb = cdiv(n, kPtT), total = nb * (nb + 1) / 2;
+  const int64_t len = cdiv(total, slots), segs = cdiv(total, len);
+  void *pc = nullptr, *pr = nullptr, *pl = nullptr;
+  GT_TRY(ws_get(WS_SCRATCH0, size_t(dist_pairs_bytes(n, dim)), &pc));
+  GT_TRY(ws_get(WS_SCRATCH1, size_t(segs + nb) * kPtT * size_t(dim + 1) * 4, &pr));
+  GT_TRY(ws_get(WS_SCRATCH2, size_t(segs) * 8, &pl));
+  PtPartials pp;
+  pp.col = static_cast<float *>(pc);
+  pp.colw = pp.col + total * kPtT * dim;
+  pp.row = static_cast<float *>(pr);
+  pp.roww = pp.row + (segs + nb) * kPtT * dim;
+  pp.loss = static_cast<double *>(pl);
+  kern<<<unsigned(segs), kPtThreads, L::BYTES, s>>>(X, n, dim, aux, nb, len, pp);
+  dist_pairs_reduce_kernel<<<unsigned(cdiv(n, kPtRedRows)), 256, 0, s>>>(X, n, dim, nb, len, pp,
+                                                                       dX);
+  count_launch(2);
+  if (MODE == 1 && loss) {
+    loss_reduce_kernel<<<1, kLossThreads, 0, s>>>(pp.loss, segs, loss);
+    count_launch();
+  }
+  GT_CUDA(cudaGetLastError());
+  return GT_OK;
+}
+
 template <int MODE>
 int launch_dist_backward(const float *X, int64_t n, int64_t dim, const float *aux, float *dX,
                          double *loss, cudaStream_t s) {
-  // measured: the tensor-core form is 10-15 % faster from 33 dimensions at 8192
-  // points and more (the fused kernel pads 33-64 dimensions to 64 and runs two
-  // CTAs per SM there), equal at 4096 points, and up to 2.5 times slower at 32
-  // dimensions and fewer.  It holds about 10 n^2 bytes of workspace, so above
-  // 32768 points (11 GB) the fused kernel, which holds none, keeps those sizes.
+  // Up to 64 dimensions each unordered pair once, while the partial sums take at
+  // most 1 GB (about 33000 points at 32 dimensions, 23000 at 64).  Measured (MDS
+  // stress, us, pairs / ordered pairs / tensor cores): 1000 x 32 24 / 34 / -,
+  // 4096 x 64 149 / 236 / 235, 8192 x 16 203 / 309 / -, 8192 x 32 296 / 455 / 670,
+  // 8192 x 48 500 / 790 / 671, 10000 x 40 720 / - / 1090.  Past that the ordered
+  // kernel holds no n^2 workspace; above 32 dimensions and up to 32768 points
+  // (11 GB there) the tensor-core form is 10-15 % faster than it, and above 64
+  // dimensions it is the only one.
+  if (dim <= 64 && dist_pairs_bytes(n, dim) <= (int64_t(1) << 30)) {
+    if (dim <= 16) return dist_backward_pairs<16, MODE>(X, n, dim, aux, dX, loss, s);
+    if (dim <= 32) return dist_backward_pairs<32, MODE>(X, n, dim, aux, dX, loss, s);
+    return dist_backward_pairs<64, MODE>(X, n, dim, aux, dX, loss, s);
+  }
   if (dim > 64 || (dim > 32 && n >= 8192 && n <= 32768))
     return dist_backward_tc<MODE>(X, n, dim, aux, dX, loss, s);
   const int64_t ib = cdiv(n, kDbRows);
