@@ -293,6 +293,55 @@ struct PearsonFinish {
     if (pairs) tc::st_stream(pp, npairs);
   }
 
+  // Whether every row of the outputs starts on a 16-byte boundary.
+  __device__ __forceinline__ bool quads() const {
+    return (ld & 3) == 0 && ((reinterpret_cast<uintptr_t>(corr) | reinterpret_cast<uintptr_t>(ts) |
+                              reinterpret_cast<uintptr_t>(pairs)) & 15) == 0;
+  }
+
+  // Whether the block has every entry and (symmetric) lies above the diagonal.
+  __device__ __forceinline__ bool interior(int64_t rbase, int64_t c0) const {
+    return (c0 + 31 < nc) && (symmetric ? (rbase + 31 < c0) : (rbase + 31 < nr));
+  }
+
+  // Four entries of one row of one orientation to the outputs at offset o.
+  __device__ __forceinline__ void put4(int64_t o, float v0, float v1, float v2, float v3) const {
+    const float4 v = make_float4(clamp_r(v0 * gscale), clamp_r(v1 * gscale), clamp_r(v2 * gscale),
+                                 clamp_r(v3 * gscale));
+    if (corr) tc::st_stream4(corr + o, v);
+    if (ts)
+      tc::st_stream4(ts + o, make_float4(signif_fast(v.x, sq_nm2), signif_fast(v.y, sq_nm2),
+                                         signif_fast(v.z, sq_nm2), signif_fast(v.w, sq_nm2)));
+    if (pairs) tc::st_stream4(pairs + o, make_float4(npairs, npairs, npairs, npairs));
+  }
+
+  // An interior block of outputs with 16-byte rows, 16 bytes a lane: a store is
+  // four 128-byte lines, and a quarter as many of them and of their addresses
+  // are issued (batch of 300 problems: 2.24 -> 2.01 ms).  Lane (row, q) takes four
+  // neighbours of row 4 k + row; the tile's odd stride keeps its reads free of
+  // bank conflicts in both orientations.
+  __device__ __forceinline__ void block_quads(int64_t rbase, int64_t c0, const float *wsm) const {
+    const int lane = threadIdx.x & 31, row = lane >> 3, q = 4 * (lane & 7);
+    if (symmetric) {
+      int64_t o = (c0 + row) * ld + rbase + q;
+      const float *w = wsm + q * 33 + row;  // entry (q + e, row + k)
+#pragma unroll 2
+      for (int k = 0; k < 32; k += 4) {
+        put4(o, w[k], w[33 + k], w[66 + k], w[99 + k]);
+        o += 4 * ld;
+      }
+    }
+    int64_t o = (rbase + row) * ld + c0 + q;
+    const float *w = wsm + row * 33 + q;  // entry (row + k, q + e)
+#pragma unroll 2
+    for (int k = 0; k < 32; k += 4) {
+      put4(o, w[0], w[1], w[2], w[3]);
+      w += 4 * 33;
+      o += 4 * ld;
+    }
+    __syncwarp();
+  }
+
   // A block from registers: g[j] = entry (r, c0 + j), lanes on consecutive rows.
   __device__ void operator()(int64_t r, int64_t c0, const float (&g)[32], EpiCtx &ctx) const {
     const int lane = threadIdx.x & 31;
@@ -318,9 +367,11 @@ struct PearsonFinish {
     const int lane = threadIdx.x & 31;
     const float *wsm = ctx.wsm;
     const int64_t rbase = r - lane;
-    // interior block: every entry exists and (symmetric) lies above the diagonal
-    const bool interior = (c0 + 31 < nc) && (symmetric ? (rbase + 31 < c0) : (rbase + 31 < nr));
-    if (interior) {
+    if (interior(rbase, c0)) {
+      if (quads()) {
+        block_quads(rbase, c0, wsm);
+        return;
+      }
       if (symmetric) {
         // mirror orientation: lanes hold consecutive rows of column c0 + j
         const int64_t o = c0 * ld + r;
