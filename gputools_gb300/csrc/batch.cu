@@ -313,12 +313,24 @@ int pearson_batch_plan(const gt_cor_problem *probs, int64_t count, int flags,
   const TileConfig *cands = x6 ? kX6Configs : kX3Configs;
   const int ncand = x6 ? int(sizeof(kX6Configs) / sizeof(kX6Configs[0]))
                        : int(sizeof(kX3Configs) / sizeof(kX3Configs[0]));
-  double work = 0.0;
-  for (int64_t i = 0; i < count; i++) work += double(probs[i].p) * double(probs[i].p) * double(probs[i].n);
+  double work = 0.0, entries = 0.0;
+  bool sectors = true;  // every output row starts on a 32-byte sector
+  for (int64_t i = 0; i < count; i++) {
+    const double e = double(probs[i].p) * double(probs[i].p);
+    entries += e;
+    work += e * double(probs[i].n);
+    sectors &= ((probs[i].ld != 0 ? probs[i].ld : probs[i].p) & 7) == 0;
+  }
   char key[128];
   std::snprintf(key, sizeof(key), "pearson:%s:%lld:%.3e", kind_name(path), (long long)count,
                 work);
-  int choice = 0;
+  // Without a tuned choice: 32-wide K blocks with their sixteen epilogue warps for
+  // the batches that their outputs bound, up to 400 observations an entry on
+  // sector-aligned rows.  Measured (us, 64-wide / 32-wide): 300 problems of up to
+  // 1024 variables x 1000 observations 338 / 313, 20 of 4096 x 200 125 / 112, 60 of
+  // 4096 x 1000 409 / 399; past it 300 of 4096 x 2000 2015 / 2056; unaligned rows
+  // 2980 / 3150.
+  int choice = !x6 && sectors && work <= 400.0 * entries ? 1 : 0;
   if (flags & GT_BATCH_AUTOTUNE) {
     gt_batch_plan *best = nullptr;
     double best_ms = 0.0;
