@@ -234,7 +234,8 @@ int launch_colstats(const float *dX, int64_t nvar, int64_t n, int use, ColStats 
 
 // prologue for the tensor-core path lives in gram_tc.cu
 int pearson_tc_prologue(const float *dX, int64_t nvar, int64_t n, int kind, int slot_z,
-                        int slot_st, void **Z, int64_t *kpad, cudaStream_t s);
+                        int slot_st, void **Z, int64_t *kpad, cudaStream_t s,
+                        const int *skip_if = nullptr);
 
 int pearson_impl(int use, const float *dA, int64_t nA, const float *dB, int64_t nB, int64_t n,
                  float *pairs, float *corr, float *ts, int symmetric, cudaStream_t s) {
@@ -258,9 +259,9 @@ int pearson_impl(int use, const float *dA, int64_t nA, const float *dB, int64_t 
   if (tc) {
     void *zA = nullptr, *zB = nullptr;
     int64_t kpad = 0;
-    GT_TRY(pearson_tc_prologue(dA, nA, n, path, WS_SCRATCH0, WS_SCRATCH2, &zA, &kpad, s));
+    GT_TRY(pearson_tc_prologue(dA, nA, n, path, WS_SCRATCH0, WS_SCRATCH2, &zA, &kpad, s, nan_flag));
     if (symmetric) zB = zA;
-    else GT_TRY(pearson_tc_prologue(dB, nB, n, path, WS_SCRATCH1, WS_SCRATCH3, &zB, &kpad, s));
+    else GT_TRY(pearson_tc_prologue(dB, nB, n, path, WS_SCRATCH1, WS_SCRATCH3, &zB, &kpad, s, nan_flag));
     GT_TRY(pearson_tc(zA, nA, zB, nB, kpad, path, po, s));
     if (use == GT_EVERYTHING) return GT_OK;
     // with a missing value: the masked tensor-core Gram (pairwise_tc.cu)

@@ -373,7 +373,8 @@ struct PairCenterer {
 // a NaN or without variance gets NaN digits, so every r involving it is NaN.
 __global__ void __launch_bounds__(256)
 pearson_exact_prep_kernel(const float *__restrict__ X, int64_t nvar, int64_t n, int64_t kpad,
-                          uint16_t *__restrict__ Z) {
+                          uint16_t *__restrict__ Z, const int *skip_if) {
+  if (skip_if && *skip_if) return;  // the Gram that reads the planes skips too
   const int64_t v = (int64_t(blockIdx.x) * 256 + threadIdx.x) >> 5;
   if (v >= nvar) return;  // whole warps
   const int lane = threadIdx.x & 31;
@@ -420,7 +421,7 @@ pearson_exact_prep_kernel(const float *__restrict__ X, int64_t nvar, int64_t n, 
 }  // namespace
 
 int pearson_exact_prologue(const float *dX, int64_t nvar, int64_t n, int slot_z, void **Z,
-                           int64_t *kpad, cudaStream_t s) {
+                           int64_t *kpad, cudaStream_t s, const int *skip_if) {
   *kpad = cdiv(n, kKPad) * kKPad;
   void *pz = nullptr;
   GT_TRY(ws_get(slot_z, size_t(kXPlanes) * size_t(nvar) * size_t(*kpad) * 2, &pz));
@@ -428,7 +429,7 @@ int pearson_exact_prologue(const float *dX, int64_t nvar, int64_t n, int slot_z,
   if (blocks > 2147483647LL) return fail(GT_EINVAL, "too many variables");
   ProfScope prof("pearson_prologue", s);
   pearson_exact_prep_kernel<<<unsigned(blocks), 256, 0, s>>>(dX, nvar, n, *kpad,
-                                                              static_cast<uint16_t *>(pz));
+                                                              static_cast<uint16_t *>(pz), skip_if);
   count_launch();
   GT_CUDA(cudaGetLastError());
   *Z = pz;

@@ -1024,7 +1024,8 @@ __device__ __forceinline__ void pearson_row(const float *__restrict__ x, int64_t
 template <int KIND>
 __global__ void __launch_bounds__(256)
 pearson_prep_kernel(const float *__restrict__ X, int64_t nvar, int64_t n, int64_t kpad,
-                    uint16_t *__restrict__ Z, ColStats *__restrict__ st) {
+                    uint16_t *__restrict__ Z, ColStats *__restrict__ st, const int *skip_if) {
+  if (skip_if && *skip_if) return;  // the Gram that reads the planes skips too
   const int64_t v = (int64_t(blockIdx.x) * 256 + threadIdx.x) >> 5;
   if (v >= nvar) return;  // whole warps
   const float *x = X + v * n;
@@ -1476,8 +1477,10 @@ int gemm_tc_store_scaled(const void *planesA, int64_t nA, const void *planesB, i
 }
 
 int pearson_tc_prologue(const float *dX, int64_t nvar, int64_t n, int kind, int slot_z,
-                        int slot_st, void **Z, int64_t *kpad, cudaStream_t s) {
-  if (kind == tc::KIND_F16X6) return pearson_exact_prologue(dX, nvar, n, slot_z, Z, kpad, s);
+                        int slot_st, void **Z, int64_t *kpad, cudaStream_t s,
+                        const int *skip_if) {
+  if (kind == tc::KIND_F16X6)
+    return pearson_exact_prologue(dX, nvar, n, slot_z, Z, kpad, s, skip_if);
   GT_TRY(check_kind(kind));
   *kpad = cdiv(n, kKPad) * kKPad;
   void *pz = nullptr, *pst = nullptr;
@@ -1489,11 +1492,14 @@ int pearson_tc_prologue(const float *dX, int64_t nvar, int64_t n, int kind, int 
   if (blocks > 2147483647LL) return fail(GT_EINVAL, "too many variables");
   ProfScope prof("pearson_prologue", s);
   if (kind == tc::KIND_BF16X6)
-    pearson_prep_kernel<tc::KIND_BF16X6><<<unsigned(blocks), 256, 0, s>>>(dX, nvar, n, *kpad, z, st);
+    pearson_prep_kernel<tc::KIND_BF16X6><<<unsigned(blocks), 256, 0, s>>>(dX, nvar, n, *kpad, z, st,
+                                                                          skip_if);
   else if (kind == tc::KIND_F16X3)
-    pearson_prep_kernel<tc::KIND_F16X3><<<unsigned(blocks), 256, 0, s>>>(dX, nvar, n, *kpad, z, st);
+    pearson_prep_kernel<tc::KIND_F16X3><<<unsigned(blocks), 256, 0, s>>>(dX, nvar, n, *kpad, z, st,
+                                                                          skip_if);
   else
-    pearson_prep_kernel<tc::KIND_BF16X3><<<unsigned(blocks), 256, 0, s>>>(dX, nvar, n, *kpad, z, st);
+    pearson_prep_kernel<tc::KIND_BF16X3><<<unsigned(blocks), 256, 0, s>>>(dX, nvar, n, *kpad, z, st,
+                                                                          skip_if);
   count_launch();
   GT_CUDA(cudaGetLastError());
   *Z = pz;

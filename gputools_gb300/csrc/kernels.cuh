@@ -69,8 +69,9 @@ int pearson_fma(const float *dA, int64_t nA, const float *dB, int64_t nB, int64_
 // prologue writes three fixed-point fp16 digit planes per variable
 // ([plane][variable][kpad], kpad a multiple of 64), the Gram sums their
 // products exactly in three TMEM accumulators, fused Pearson epilogue.
+// With skip_if, the prologue does nothing where *skip_if != 0 (a device flag).
 int pearson_exact_prologue(const float *dX, int64_t nvar, int64_t n, int slot_z, void **Z,
-                           int64_t *kpad, cudaStream_t s);
+                           int64_t *kpad, cudaStream_t s, const int *skip_if = nullptr);
 int pearson_exact(const void *zA, int64_t nA, const void *zB, int64_t nB, int64_t kpad,
                   const PearsonOut &out, cudaStream_t s);
 // The Pearson Gram on a device table of tiles (row0, col0) of 128 x 256 (see
