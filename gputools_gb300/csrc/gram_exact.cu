@@ -35,12 +35,12 @@
 // lies wholly below the diagonal of a symmetric problem is skipped).  Problems
 // that fill the chip with 256 x 256 tiles run them on pairs of CTAs
 // (cta_group::2, clusters of two): the halves are 256 x 128, each CTA holding 128
-// rows of A and 64 of B, so a stage fetches a quarter less.  What bounds both
-// is the power limit: with the operands left in place (no copies at all) the
-// MMAs alone take 6.0 ms of the 6.4 that the pairs take at 20000 x 4096 (1.53
-// PFLOP/s; cuBLAS holds 1.71 under the cap), 6.7 before pairs and 128-byte rows.
+// rows of A and 64 of B, so a stage fetches a quarter less.  20000 x 4096: 5.9 ms
+// (1.66 PFLOP/s; cuBLAS holds 1.71 under the power limit), 6.7 on single CTAs
+// with one lane issuing from a branch.  With the operands left in place (no
+// copies) the MMAs alone take 4.7: the copies' latency bounds it.
 //   warp 0      TMA producer: 3-D loads of the three digit planes of the A
-//               (128-row) and B (128- or 64-row) boxes, 64 k per stage;
+//               (128-row) and B (128- or 64-row) boxes, 32 k per stage;
 //   warp 1      allocates 512 TMEM columns (three 128 x 128 accumulators) and
 //               one thread issues six tcgen05.mma (M = 128, N = 128, K = 16)
 //               per k-step: P0.P0 -> S0, P0.X1, X1.P0 -> S1,
@@ -64,10 +64,10 @@ namespace gt {
 namespace {
 
 constexpr int kXB = 128;     // columns of a half tile (MMA N)
-// k per stage: 128-byte rows with the 128-byte swizzle.  Two stages of 64 take
-// 6.91 ms at 20000 x 4096 where five of 32 take 7.21 (pairs; 7.07 and 7.35 single):
-// half as many rows to fetch.
-constexpr int kXBK = 64;
+// k per stage (64-byte rows, 64-byte swizzle): five stages of 32 take 6.20 ms at
+// 20000 x 4096 where two of 64 take 6.69 (pairs): the copies' latency is what
+// the stages have to cover.
+constexpr int kXBK = 32;
 constexpr int kXPlanes = 3;  // digit planes P0, X1, X2
 constexpr int kXEpi = 8;     // epilogue warps
 constexpr int kXThreads = 64 + 32 * kXEpi;
@@ -143,34 +143,37 @@ gram_exact_kernel(const __grid_constant__ Work work, const tc::WaitCfg wc) {
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
-      // ------------------------------------------------ TMA producer
-      int64_t it = 0;
-      TileRef ref;
-      TileCursor<Work> tiles(work, 0, 1);
-      bool go = true;
-      while (go && !*abort_flag && tiles.next(ref)) {
-        const auto &fin = work.finish(ref);
-        for (int h = 0; h < 2 && go; h++) {
-          if (!half_live(fin, ref, h)) continue;
-          const int32_t r0 = int32_t(ref.row0) + rank * kBM;
-          const int32_t c0 = int32_t(ref.col0 + int64_t(h) * kXB) + rank * C::BROWS;
-          for (int64_t kb = 0; kb < ref.nk; kb++, it++) {
-            const int s = int(it % kXStages);
-            const uint32_t use = uint32_t(it / kXStages);
-            if (!tc::mbar_wait(&empty[s], (use & 1u) ^ 1u, abort_flag, wc)) {
-              *abort_flag = 1;
-              go = false;
-              break;
-            }
-            uint8_t *st = smem + s * kXStage;
+    // -------------------------------------------------- TMA producer
+    // (the whole warp walks the loop, one elected lane issues, as below)
+    int it = 0;
+    const bool lead = tc::elect_one();
+    TileRef ref;
+    TileCursor<Work> tiles(work, 0, 1);
+    bool go = true;
+    while (go && !*abort_flag && tiles.next(ref)) {
+      const auto &fin = work.finish(ref);
+      const int nk = int(ref.nk);
+      for (int h = 0; h < 2 && go; h++) {
+        if (!half_live(fin, ref, h)) continue;
+        const int32_t r0 = int32_t(ref.row0) + rank * kBM;
+        const int32_t c0 = int32_t(ref.col0) + h * kXB + rank * C::BROWS;
+        for (int kb = 0; kb < nk; kb++, it++) {
+          const int s = it % kXStages;
+          go = __all_sync(0xffffffffu, tc::mbar_wait(&empty[s], (uint32_t(it / kXStages) & 1u) ^ 1u,
+                                                     abort_flag, wc));
+          if (!go) {
+            *abort_flag = 1;
+            break;
+          }
+          uint8_t *st = smem + s * kXStage;
+          if (lead) {
             // a pair's copies all count on the even CTA's barrier
             if (rank == 0) tc::mbar_arrive_expect_tx(&full[s], (PAIR ? 2 : 1) * kXStage);
             auto load = [&](void *dst, const CUtensorMap *map, int32_t row, int p) {
               if constexpr (PAIR)
-                tc::tma_load_3d_pair(dst, map, &full[s], int32_t(kb * kXBK), row, p);
+                tc::tma_load_3d_pair(dst, map, &full[s], kb * kXBK, row, p);
               else
-                tc::tma_load_3d(dst, map, &full[s], int32_t(kb * kXBK), row, p);
+                tc::tma_load_3d(dst, map, &full[s], kb * kXBK, row, p);
             };
 #pragma unroll
             for (int p = 0; p < kXPlanes; p++) load(st + p * kXATile, ref.ma, r0, p);
@@ -178,55 +181,55 @@ gram_exact_kernel(const __grid_constant__ Work work, const tc::WaitCfg wc) {
             for (int p = 0; p < kXPlanes; p++)
               load(st + kXPlanes * kXATile + p * kXBTile, ref.mb, c0, p);
           }
+          __syncwarp();
         }
       }
-      // drain: no bulk copy may still be writing shared memory at exit
-      // (a pair that gives up lets time pass below instead)
-      if (!PAIR && *abort_flag) {
-        for (int s = 0; s < kXStages; s++) {
-          const int64_t fills = it / kXStages + (s < it % kXStages ? 1 : 0);
-          if (fills > 0) tc::mbar_wait_bounded(&full[s], uint32_t((fills - 1) & 1), kDrainLimitNs);
-        }
+    }
+    // drain: no bulk copy may still be writing shared memory at exit
+    // (a pair that gives up lets time pass below instead)
+    if (!PAIR && *abort_flag && lead) {
+      for (int s = 0; s < kXStages; s++) {
+        const int fills = it / kXStages + (s < it % kXStages ? 1 : 0);
+        if (fills > 0) tc::mbar_wait_bounded(&full[s], uint32_t((fills - 1) & 1), kDrainLimitNs);
       }
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ------------------------------------------------ MMA issuer
-      // of a pair: the even CTA's thread
-      constexpr uint32_t idesc = tc::idesc_f32acc(PAIR ? 2 * kBM : kBM, kXB, 0u /* fp16 */);
-      int64_t it = 0, hc = 0;
-      bool ok = true;
-      TileRef ref;
-      TileCursor<Work> tiles(work, 0, 1);
-      while (rank == 0 && ok && tiles.next(ref)) {
-        const auto &fin = work.finish(ref);
-        for (int h = 0; h < 2 && ok; h++) {
-          if (!half_live(fin, ref, h)) continue;
-          // the epilogue has read the previous half's sums
-          if (!tc::mbar_wait(acce, uint32_t(hc & 1) ^ 1u, abort_flag, wc)) {
-            ok = false;
-            break;
-          }
+    // -------------------------------------------------- MMA issuer
+    // (of a pair: the even CTA's).  The whole warp walks the loop, so that the
+    // addresses stay in uniform registers; one elected lane issues.
+    constexpr uint32_t idesc = tc::idesc_f32acc(PAIR ? 2 * kBM : kBM, kXB, 0u /* fp16 */);
+    int it = 0, hc = 0;
+    bool ok = true;
+    const bool lead = tc::elect_one();
+    TileRef ref;
+    TileCursor<Work> tiles(work, 0, 1);
+    while (rank == 0 && ok && tiles.next(ref)) {
+      const auto &fin = work.finish(ref);
+      const int nk = int(ref.nk);
+      for (int h = 0; h < 2 && ok; h++) {
+        if (!half_live(fin, ref, h)) continue;
+        // the epilogue has read the previous half's sums
+        ok = __all_sync(0xffffffffu, tc::mbar_wait(acce, uint32_t(hc & 1) ^ 1u, abort_flag, wc));
+        if (!ok) break;
+        tc::tc_fence_after();
+        for (int kb = 0; kb < nk; kb++, it++) {
+          const int s = it % kXStages;
+          ok = __all_sync(0xffffffffu, tc::mbar_wait(&full[s], uint32_t(it / kXStages) & 1u,
+                                                     abort_flag, wc));
+          if (!ok) break;
           tc::tc_fence_after();
-          for (int64_t kb = 0; kb < ref.nk; kb++, it++) {
-            const int s = int(it % kXStages);
-            const uint32_t use = uint32_t(it / kXStages);
-            if (!tc::mbar_wait(&full[s], use & 1u, abort_flag, wc)) {
-              ok = false;
-              break;
-            }
-            tc::tc_fence_after();
-            const uint32_t sa = tc::smem_u32(smem + s * kXStage);
-            const uint32_t sb = sa + kXPlanes * kXATile;
+          const uint32_t sa = tc::smem_u32(smem + s * kXStage);
+          const uint32_t sb = sa + kXPlanes * kXATile;
+          if (lead) {
 #pragma unroll
             for (int k = 0; k < kXBK / 16; k++) {
 #pragma unroll
               for (int p = 0; p < 6; p++) {
                 int pa, pb, acc;
                 exact_product(p, pa, pb, acc);
-                const uint64_t ad = tc::smem_desc_kmajor(sa + pa * kXATile + k * 32, 128);
-                const uint64_t bd = tc::smem_desc_kmajor(sb + pb * kXBTile + k * 32, 128);
+                const uint64_t ad = tc::smem_desc_kmajor(sa + pa * kXATile + k * 32, 64);
+                const uint64_t bd = tc::smem_desc_kmajor(sb + pb * kXBTile + k * 32, 64);
                 // the first product into each sum starts it
                 const uint32_t more = kb == 0 && k == 0 && (p == 0 || p == 1 || p == 3) ? 0u : 1u;
                 if constexpr (PAIR)
@@ -238,14 +241,20 @@ gram_exact_kernel(const __grid_constant__ Work work, const tc::WaitCfg wc) {
             if constexpr (PAIR) tc::umma_commit_pair(&empty[s]);
             else tc::umma_commit(&empty[s]);
           }
-          if (!ok) break;
+          __syncwarp();
+        }
+        if (!ok) break;
+        if (lead) {
           if constexpr (PAIR) tc::umma_commit_pair(accf);
           else tc::umma_commit(accf);
-          hc++;
         }
+        __syncwarp();
+        hc++;
       }
-      if (!ok) *abort_flag = 1;
-      // every MMA issued above has finished before TMEM is released
+    }
+    if (!ok) *abort_flag = 1;
+    // every MMA issued above has finished before TMEM is released
+    if (lead) {
       if constexpr (PAIR) {
         if (rank == 0) tc::umma_commit_pair(mma_done);
       } else {
@@ -497,8 +506,8 @@ int pearson_exact(const void *zA, int64_t nA, const void *zB, int64_t nB, int64_
   if (!out.corr && !out.ts && !out.pairs) return GT_OK;
   if (kpad <= 0 || kpad % kKPad) return fail(GT_EINVAL, "bad padded K (%lld)", (long long)kpad);
   const int64_t panel = int64_t(kBN) * kpad * 2 * kXPlanes;
-  // pairs: twice as wide bands, measured with 8 / 16 / 32 / 64 panels of 6 MB 6.98 /
-  // 6.82 / 6.88 / 7.04 ms
+  // pairs: twice as wide bands, measured with 4 / 8 / 16 / 32 panels of 6 MB 6.48 /
+  // 6.26 / 6.20 / 6.31 ms
   const PairSpace ps = make_pair_space(nA, nB, out.symmetric, band_group(panel / 2));
   // at least one tile for every pair; below that single CTAs' smaller tiles
   // spread better

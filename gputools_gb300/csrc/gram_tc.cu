@@ -587,7 +587,8 @@ struct StoreFinish {
 // memory to the stages.
 // WIDE: sixteen epilogue warps of 64 columns for a chunked kernel (the
 // Pearson finish, whose stores are latency-bound at two warps per scheduler).
-template <int KIND, int BK, bool LISTS, bool WIDE = false>
+// PAIR: CTA pairs on 256 x 256 tiles, each CTA with 128 rows of A and of B.
+template <int KIND, int BK, bool LISTS, bool WIDE = false, bool PAIR = false>
 struct TcCfg {
   static constexpr int NSPLIT = tc::Kind<KIND>::NSPLIT;
   static constexpr int EPI = (LISTS || WIDE) ? 16 : 8;       // epilogue warps
@@ -595,7 +596,8 @@ struct TcCfg {
   static constexpr int COLS = 4 * kBN / EPI;                 // columns per epilogue warp
   static constexpr int ROW_BYTES = BK * 2;                // 128 or 64
   static constexpr int A_TILE = kBM * BK * 2;
-  static constexpr int B_TILE = kBN * BK * 2;
+  static constexpr int BROWS = PAIR ? kBN / 2 : kBN;      // B rows that this CTA loads
+  static constexpr int B_TILE = BROWS * BK * 2;
   static constexpr int STAGE = NSPLIT * (A_TILE + B_TILE);
   static constexpr int EPI_FLOATS = kEpiTileFloats + (LISTS ? kEuclidList + 2 * COLS : 0);
   static constexpr int EPI_BYTES = EPI * EPI_FLOATS * 4;
@@ -714,15 +716,20 @@ struct wide_epi<Work, std::void_t<decltype(Work::kWideEpi)>>
 // outputs are pitched, and on sector-aligned rows the extra warps hide the
 // store latency (single problems with a row stride off the 32-byte sectors
 // store slower with them).
-template <int KIND, int BK, bool CHUNKED, class Work>
+template <int KIND, int BK, bool CHUNKED, class Work, bool PAIR = false>
 using KernelCfg = TcCfg<KIND, BK, !CHUNKED,
                         CHUNKED && BK == 32 && wide_epi<Work>::value &&
-                            staged_block<FinOf<Work>>::value>;
+                            staged_block<FinOf<Work>>::value,
+                        PAIR>;
 
-template <int KIND, int BK, bool CHUNKED, class Work>
-__global__ void __launch_bounds__(KernelCfg<KIND, BK, CHUNKED, Work>::THREADS, 1)
+// PAIR: clusters of two CTAs (cta_group::2), tiles of 256 x 256 whose row0 is the
+// pair's; the even CTA issues the MMAs, both CTAs' copies count on its barriers.
+// A 128 x 256 tile needs 64 bytes per tensor-core cycle from L2 (f16x3), more
+// than the 42 or so that an SM gets; a pair needs 43.
+template <int KIND, int BK, bool CHUNKED, class Work, bool PAIR = false>
+__global__ void __launch_bounds__(KernelCfg<KIND, BK, CHUNKED, Work, PAIR>::THREADS, 1)
 gram_tc_kernel(const __grid_constant__ Work work, int64_t ckb, const tc::WaitCfg wc) {
-  using C = KernelCfg<KIND, BK, CHUNKED, Work>;
+  using C = KernelCfg<KIND, BK, CHUNKED, Work, PAIR>;
   if (work.skip()) return;  // a gated launch whose gate is closed: before any setup
   constexpr int NSPLIT = C::NSPLIT;
   static_assert(!CHUNKED || C::COLS == 128 || C::COLS == 64,
@@ -741,6 +748,7 @@ gram_tc_kernel(const __grid_constant__ Work work, int64_t ckb, const tc::WaitCfg
   float *epi_smem = reinterpret_cast<float *>(smem + C::STAGES * C::STAGE + 256);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = PAIR ? int(tc::cluster_rank()) : 0;
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; s++) {
       tc::mbar_init(&full[s], 1);
@@ -748,85 +756,98 @@ gram_tc_kernel(const __grid_constant__ Work work, int64_t ckb, const tc::WaitCfg
     }
     for (int b = 0; b < 2; b++) {
       tc::mbar_init(&accf[b], 1);
-      tc::mbar_init(&acce[b], C::EPI);
+      tc::mbar_init(&acce[b], PAIR ? 2 * C::EPI : C::EPI);
     }
     tc::mbar_init(mma_done, 1);
     *abort_flag = 0;
     tc::fence_barrier_init();
   }
   if (warp == 0 && lane == 0) work.prefetch();
-  if (warp == 1) tc::tmem_alloc(tmem_slot, 2 * kBN);
+  if (warp == 1) tc::tmem_alloc<PAIR>(tmem_slot, 2 * kBN);
   tc::tc_fence_before();
   __syncthreads();
+  if constexpr (PAIR) tc::cluster_sync();  // both CTAs' barriers and TMEM are there
   tc::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == 0) {
-    if (lane == 0) {
-      // ------------------------------------------------ TMA producer
-      int64_t it = 0;
-      TileRef ref;
-      TileCursor<Work> tiles(work, 0, 1);
-      while (!*abort_flag && tiles.next(ref)) {
-        for (int64_t kb = 0; kb < ref.nk; kb++, it++) {
-          const int s = int(it % C::STAGES);
-          const uint32_t use = uint32_t(it / C::STAGES);
-          if (!tc::mbar_wait(&empty[s], (use & 1u) ^ 1u, abort_flag, wc)) {
-            *abort_flag = 1;
-            break;
-          }
-          uint8_t *st = smem + s * C::STAGE;
-          tc::mbar_arrive_expect_tx(&full[s], C::STAGE);
-#pragma unroll
-          for (int p = 0; p < NSPLIT; p++)
-            tc::tma_load_3d(st + p * C::A_TILE, ref.ma, &full[s], int32_t((ref.k0 + kb) * BK),
-                            int32_t(ref.row0), p);
-#pragma unroll
-          for (int p = 0; p < NSPLIT; p++)
-            tc::tma_load_3d(st + NSPLIT * C::A_TILE + p * C::B_TILE, ref.mb, &full[s],
-                            int32_t((ref.k0 + kb) * BK), int32_t(ref.col0), p);
+    // -------------------------------------------------- TMA producer
+    // (the whole warp walks the loop, one elected lane issues, as below)
+    int it = 0;
+    const bool lead = tc::elect_one();
+    bool go = true;
+    TileRef ref;
+    TileCursor<Work> tiles(work, 0, 1);
+    while (go && !*abort_flag && tiles.next(ref)) {
+      const int nk = int(ref.nk), k0 = int(ref.k0);
+      const int32_t r0 = int32_t(ref.row0) + rank * kBM, c0 = int32_t(ref.col0) + rank * C::BROWS;
+      for (int kb = 0; kb < nk; kb++, it++) {
+        const int s = it % C::STAGES;
+        go = __all_sync(0xffffffffu, tc::mbar_wait(&empty[s], (uint32_t(it / C::STAGES) & 1u) ^ 1u,
+                                                   abort_flag, wc));
+        if (!go) {
+          *abort_flag = 1;
+          break;
         }
+        uint8_t *st = smem + s * C::STAGE;
+        if (lead) {
+          if (rank == 0) tc::mbar_arrive_expect_tx(&full[s], (PAIR ? 2 : 1) * C::STAGE);
+          auto load = [&](void *dst, const CUtensorMap *map, int32_t row, int p) {
+            if constexpr (PAIR) tc::tma_load_3d_pair(dst, map, &full[s], (k0 + kb) * BK, row, p);
+            else tc::tma_load_3d(dst, map, &full[s], (k0 + kb) * BK, row, p);
+          };
+#pragma unroll
+          for (int p = 0; p < NSPLIT; p++) load(st + p * C::A_TILE, ref.ma, r0, p);
+#pragma unroll
+          for (int p = 0; p < NSPLIT; p++)
+            load(st + NSPLIT * C::A_TILE + p * C::B_TILE, ref.mb, c0, p);
+        }
+        __syncwarp();
       }
-      // drain: no bulk copy may still be writing shared memory at exit
-      if (*abort_flag) {
-        for (int s = 0; s < C::STAGES; s++) {
-          const int64_t fills = it / C::STAGES + (s < it % C::STAGES ? 1 : 0);
-          if (fills > 0) tc::mbar_wait_bounded(&full[s], uint32_t((fills - 1) & 1), kDrainLimitNs);
-        }
+    }
+    // drain: no bulk copy may still be writing shared memory at exit
+    // (a pair that gives up lets time pass below instead)
+    if (!PAIR && *abort_flag && lead) {
+      for (int s = 0; s < C::STAGES; s++) {
+        const int fills = it / C::STAGES + (s < it % C::STAGES ? 1 : 0);
+        if (fills > 0) tc::mbar_wait_bounded(&full[s], uint32_t((fills - 1) & 1), kDrainLimitNs);
       }
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ------------------------------------------------ MMA issuer
-      constexpr uint32_t idesc = tc::idesc_f32acc(kBM, kBN, tc::Kind<KIND>::AB_FMT);
-      int64_t it = 0, cc = 0;
-      bool ok = true;
-      TileRef ref;
-      TileCursor<Work> tiles(work, 0, 1);
-      while (ok && tiles.next(ref)) {
-        const int64_t ck = CHUNKED ? ckb : ref.nk;
-        const int64_t nch = (ref.nk + ck - 1) / ck;
-        for (int64_t ch = 0; ch < nch && ok; ch++, cc++) {
-          const int buf = int(cc & 1);
-          const uint32_t ause = uint32_t(cc >> 1);
-          if (!tc::mbar_wait(&acce[buf], (ause & 1u) ^ 1u, abort_flag, wc)) {
-            ok = false;
-            break;
-          }
+    // -------------------------------------------------- MMA issuer
+    // The whole warp walks the loop, so that the descriptors stay in uniform
+    // registers; one elected lane issues.  (Issued from a branch of one lane,
+    // every descriptor word went through a vector register: the issue took
+    // longer than the multiply, and about 65 % of the tensor cores' rate was
+    // the limit of every kernel here.)
+    constexpr uint32_t idesc = tc::idesc_f32acc(PAIR ? 2 * kBM : kBM, kBN, tc::Kind<KIND>::AB_FMT);
+    constexpr unsigned FULLM = 0xffffffffu;
+    int it = 0, cc = 0;
+    bool ok = true;
+    const bool lead = tc::elect_one();
+    TileRef ref;
+    TileCursor<Work> tiles(work, 0, 1);
+    while (rank == 0 && ok && tiles.next(ref)) {
+      const int nk = int(ref.nk);
+      const int ck = CHUNKED ? int(ckb) : nk;
+      for (int kb0 = 0; kb0 < nk && ok; kb0 += ck, cc++) {
+        const int buf = cc & 1;
+        ok = __all_sync(FULLM, tc::mbar_wait(&acce[buf], (uint32_t(cc >> 1) & 1u) ^ 1u, abort_flag,
+                                             wc));
+        if (!ok) break;
+        tc::tc_fence_after();
+        const uint32_t d = tmem_base + uint32_t(buf * kBN);
+        const int kb1 = kb0 + ck < nk ? kb0 + ck : nk;
+        for (int kb = kb0; kb < kb1; kb++, it++) {
+          const int s = it % C::STAGES;
+          ok = __all_sync(FULLM, tc::mbar_wait(&full[s], uint32_t(it / C::STAGES) & 1u, abort_flag,
+                                               wc));
+          if (!ok) break;
           tc::tc_fence_after();
-          const uint32_t d = tmem_base + uint32_t(buf * kBN);
-          const int64_t kb0 = ch * ck, kb1 = (kb0 + ck < ref.nk) ? kb0 + ck : ref.nk;
-          for (int64_t kb = kb0; kb < kb1; kb++, it++) {
-            const int s = int(it % C::STAGES);
-            const uint32_t use = uint32_t(it / C::STAGES);
-            if (!tc::mbar_wait(&full[s], use & 1u, abort_flag, wc)) {
-              ok = false;
-              break;
-            }
-            tc::tc_fence_after();
-            const uint32_t sa = tc::smem_u32(smem + s * C::STAGE);
-            const uint32_t sb = sa + NSPLIT * C::A_TILE;
+          const uint32_t sa = tc::smem_u32(smem + s * C::STAGE);
+          const uint32_t sb = sa + NSPLIT * C::A_TILE;
+          if (lead) {
 #pragma unroll
             for (int k = 0; k < C::KSTEPS; k++) {
 #pragma unroll
@@ -835,17 +856,31 @@ gram_tc_kernel(const __grid_constant__ Work work, int64_t ckb, const tc::WaitCfg
                 product_parts<NSPLIT>(p, pa, pb);
                 const uint64_t ad = tc::smem_desc_kmajor(sa + pa * C::A_TILE + k * 32, C::ROW_BYTES);
                 const uint64_t bd = tc::smem_desc_kmajor(sb + pb * C::B_TILE + k * 32, C::ROW_BYTES);
-                tc::umma_bf16(d, ad, bd, idesc, (kb != kb0 || k || p) ? 1u : 0u);
+                const uint32_t more = (kb != kb0 || k || p) ? 1u : 0u;
+                if constexpr (PAIR) tc::umma_bf16_pair(d, ad, bd, idesc, more);
+                else tc::umma_bf16(d, ad, bd, idesc, more);
               }
             }
-            tc::umma_commit(&empty[s]);
+            if constexpr (PAIR) tc::umma_commit_pair(&empty[s]);
+            else tc::umma_commit(&empty[s]);
           }
-          if (ok) tc::umma_commit(&accf[buf]);
+          __syncwarp();
         }
+        if (ok && lead) {
+          if constexpr (PAIR) tc::umma_commit_pair(&accf[buf]);
+          else tc::umma_commit(&accf[buf]);
+        }
+        __syncwarp();
       }
-      if (!ok) *abort_flag = 1;
-      // every MMA issued above has finished before TMEM is released
-      tc::umma_commit(mma_done);
+    }
+    if (!ok) *abort_flag = 1;
+    // every MMA issued above has finished before TMEM is released
+    if (lead) {
+      if constexpr (PAIR) {
+        if (rank == 0) tc::umma_commit_pair(mma_done);
+      } else {
+        tc::umma_commit(mma_done);
+      }
       tc::mbar_wait_bounded(mma_done, 0u, kDrainLimitNs);
     }
     __syncwarp();
@@ -864,7 +899,7 @@ gram_tc_kernel(const __grid_constant__ Work work, int64_t ckb, const tc::WaitCfg
     TileCursor<Work> tiles(work, 0, 1);
     while (ok && tiles.next(ref)) {
       const auto &fin = work.finish(ref);
-      const int64_t r = ref.row0 + q * 32 + lane;
+      const int64_t r = ref.row0 + rank * kBM + q * 32 + lane;
       const int64_t col = ref.col0 + part * C::COLS;
       ctx.rbase = r - lane;
       ctx.col0 = col;
@@ -894,7 +929,10 @@ gram_tc_kernel(const __grid_constant__ Work work, int64_t ckb, const tc::WaitCfg
           }
           tc::tc_fence_before();
           __syncwarp();
-          if (lane == 0) tc::mbar_arrive(&acce[buf]);
+          if (lane == 0) {
+            if constexpr (PAIR) tc::mbar_arrive_cta(&acce[buf], 0);
+            else tc::mbar_arrive(&acce[buf]);
+          }
         }
         if (!ok) break;
         using FinT = std::decay_t<decltype(fin)>;
@@ -948,7 +986,10 @@ gram_tc_kernel(const __grid_constant__ Work work, int64_t ckb, const tc::WaitCfg
         }
         tc::tc_fence_before();
         __syncwarp();
-        if (lane == 0) tc::mbar_arrive(&acce[buf]);
+        if (lane == 0) {
+          if constexpr (PAIR) tc::mbar_arrive_cta(&acce[buf], 0);
+          else tc::mbar_arrive(&acce[buf]);
+        }
         cc++;
         fin.end_tile(ctx);
       }
@@ -958,9 +999,18 @@ gram_tc_kernel(const __grid_constant__ Work work, int64_t ckb, const tc::WaitCfg
   }
   __syncthreads();
   if (*abort_flag && threadIdx.x == 0) atomicOr(wc.err, 1);
+  if constexpr (PAIR) {
+    if (*abort_flag && threadIdx.x == 0) tc::pass_time(tc::kCopyTimeNs);
+    __syncthreads();
+    tc::cluster_sync();  // the even CTA's MMAs use both CTAs' memory and arrive in both
+  }
   if (warp == 1) {
     tc::tc_fence_after();
-    tc::tmem_dealloc(tmem_base, 2 * kBN);
+    tc::tmem_dealloc<PAIR>(tmem_base, 2 * kBN);
+  }
+  if constexpr (PAIR) {
+    __syncwarp();
+    tc::cluster_sync();
   }
 }
 
@@ -1310,6 +1360,33 @@ template <int KIND, int BK, bool CHUNKED, class Fin>
 int launch_gram(const void *zA, int64_t nA, const void *zB, int64_t nB, int64_t kpad,
                 int mode, int64_t ckb, const Fin &fin, const char *prof_name,
                 cudaStream_t s) {
+  if constexpr (CHUNKED && BK == 32) {
+    // CTA pairs on 256 x 256 tiles where every pair of SMs gets one (fewer tiles leave
+    // SMs idle that 128 x 256 ones would use).  f16x3, single CTAs against pairs:
+    // 500 observations x 2817 variables (78 tiles) 74 -> 57 us, x 10000 270 -> 263,
+    // 4096 x 20000 3766 -> 3587, mutual information of 1000 x 2000 (10 bins) 703 ->
+    // 664; where the outputs bound it, 100 x 12000, 304 -> 310.
+    const PairSpace ps = make_pair_space(nA, nB, mode == kUpper ? 1 : 0,
+                                         band_group(int64_t(kBN) * kpad * tc::Kind<KIND>::NSPLIT));
+    if (2 * ps.ntiles >= sm_count() && ps.ntiles <= 2147483647LL && nA > kBM && mode != kLower &&
+        kpad > 0 && kpad % kKPad == 0) {
+      using PC = TcCfg<KIND, BK, false, false, true>;
+      PairWork<Fin> w;
+      GT_TRY(make_plane_map(&w.ma, zA, nA, kpad, PC::NSPLIT, kBM, BK, tc::Kind<KIND>::F16));
+      GT_TRY(make_plane_map(&w.mb, zB, nB, kpad, PC::NSPLIT, PC::BROWS, BK, tc::Kind<KIND>::F16));
+      w.ps = ps;
+      w.nk = kpad / BK;
+      w.fin = fin;
+      tc::WaitCfg wc;
+      GT_TRY(make_wait_cfg(&wc));
+      auto kern = gram_tc_kernel<KIND, BK, true, PairWork<Fin>, true>;
+      using KC = KernelCfg<KIND, BK, true, PairWork<Fin>, true>;
+      GT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, KC::SMEM));
+      ProfScope prof(prof_name, s);
+      return launch_pairs(kern, ps.ntiles, KC::THREADS, KC::SMEM, s, w, ckb < 1 ? int64_t(1) : ckb,
+                          wc);
+    }
+  }
   using C = TcCfg<KIND, BK, !CHUNKED>;
   using W = SingleWork<Fin>;
   constexpr bool F16 = tc::Kind<KIND>::F16;

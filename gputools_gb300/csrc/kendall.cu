@@ -312,25 +312,29 @@ kendall_gram_kernel(const __grid_constant__ CUtensorMap ma, const __grid_constan
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = tc::idesc_e4m3_f32acc(kBM, kBN);
-      bool ok = true;
-      for (int it = 0; it < nk; it++) {
-        const int s = it % kSgStages;
-        if (!tc::mbar_wait(&full[s], uint32_t((it / kSgStages) & 1), abort_flag, wc)) {
-          ok = false;
-          break;
-        }
-        tc::tc_fence_after();
-        const uint32_t sa = tc::smem_u32(smem + s * kSgStage), sb = sa + kSgATile;
+    // the whole warp walks the loop (descriptors in uniform registers), one lane issues
+    constexpr uint32_t idesc = tc::idesc_e4m3_f32acc(kBM, kBN);
+    const bool lead = tc::elect_one();
+    bool ok = true;
+    for (int it = 0; it < nk; it++) {
+      const int s = it % kSgStages;
+      ok = __all_sync(0xffffffffu, tc::mbar_wait(&full[s], uint32_t((it / kSgStages) & 1),
+                                                 abort_flag, wc));
+      if (!ok) break;
+      tc::tc_fence_after();
+      const uint32_t sa = tc::smem_u32(smem + s * kSgStage), sb = sa + kSgATile;
+      if (lead) {
 #pragma unroll
         for (int k = 0; k < kSgBK / 32; k++)
           tc::umma_f8(tmem, tc::smem_desc_kmajor(sa + k * 32, 128),
                       tc::smem_desc_kmajor(sb + k * 32, 128), idesc, it == 0 && k == 0 ? 0u : 1u);
         tc::umma_commit(&empty[s]);
       }
-      if (!ok) *abort_flag = 1;
-      // every MMA issued above has finished before the sums are read and TMEM is released
+      __syncwarp();
+    }
+    if (!ok) *abort_flag = 1;
+    // every MMA issued above has finished before the sums are read and TMEM is released
+    if (lead) {
       tc::umma_commit(done);
       if (!ok) tc::mbar_wait_bounded(done, 0u, kDrainLimitNs);
     }

@@ -206,36 +206,37 @@ pairwise_tc_kernel(const __grid_constant__ PairwiseArgs a, const tc::WaitCfg wc)
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
-      // ------------------------------------------------ MMA issuer
-      constexpr uint32_t id160 = tc::idesc_f32acc(kPM, 160, 0);
-      constexpr uint32_t id64 = tc::idesc_f32acc(kPM, 64, 0);
-      constexpr uint32_t id32 = tc::idesc_f32acc(kPM, 32, 0);
-      int64_t it = 0, cc = 0;
-      bool ok = true;
-      for (int64_t t = blockIdx.x; t < a.ntiles && ok; t += gridDim.x) {
-        for (int64_t ch = 0; ch < nch && ok; ch++, cc++) {
-          // two accumulator sets: wait until the epilogue has read the set's
-          // previous chunk
-          const int buf = int(cc & 1);
-          if (!tc::mbar_wait(&acce[buf], uint32_t((cc >> 1) & 1) ^ 1u, abort_flag, wc)) {
-            ok = false;
-            break;
-          }
+    // -------------------------------------------------- MMA issuer
+    // (the whole warp walks the loop, so that the descriptors stay in uniform
+    // registers; one elected lane issues)
+    constexpr uint32_t id160 = tc::idesc_f32acc(kPM, 160, 0);
+    constexpr uint32_t id64 = tc::idesc_f32acc(kPM, 64, 0);
+    constexpr uint32_t id32 = tc::idesc_f32acc(kPM, 32, 0);
+    constexpr unsigned FULLM = 0xffffffffu;
+    const int nk = int(a.nk);
+    int it = 0, cc = 0;
+    bool ok = true;
+    const bool lead = tc::elect_one();
+    for (int64_t t = blockIdx.x; t < a.ntiles && ok; t += gridDim.x) {
+      for (int kb0 = 0; kb0 < nk && ok; kb0 += int(kPChunkKb), cc++) {
+        // two accumulator sets: wait until the epilogue has read the set's
+        // previous chunk
+        const int buf = cc & 1;
+        ok = __all_sync(FULLM, tc::mbar_wait(&acce[buf], uint32_t((cc >> 1) & 1) ^ 1u, abort_flag,
+                                             wc));
+        if (!ok) break;
+        tc::tc_fence_after();
+        const uint32_t d = tmem_base + uint32_t(buf * kPAcc);
+        const int kb1 = kb0 + int(kPChunkKb) < nk ? kb0 + int(kPChunkKb) : nk;
+        for (int kb = kb0; kb < kb1; kb++, it++) {
+          const int s = it % kPStages;
+          ok = __all_sync(FULLM, tc::mbar_wait(&full[s], uint32_t(it / kPStages) & 1u, abort_flag,
+                                               wc));
+          if (!ok) break;
           tc::tc_fence_after();
-          const uint32_t d = tmem_base + uint32_t(buf * kPAcc);
-          const int64_t kb0 = ch * kPChunkKb;
-          const int64_t kb1 = kb0 + kPChunkKb < a.nk ? kb0 + kPChunkKb : a.nk;
-          for (int64_t kb = kb0; kb < kb1; kb++, it++) {
-            const int s = int(it % kPStages);
-            const uint32_t use = uint32_t(it / kPStages);
-            if (!tc::mbar_wait(&full[s], use & 1u, abort_flag, wc)) {
-              ok = false;
-              break;
-            }
-            tc::tc_fence_after();
-            const uint32_t sa = tc::smem_u32(smem + s * kPStage);
-            const uint32_t sb = sa + kPlanes * kPA;
+          const uint32_t sa = tc::smem_u32(smem + s * kPStage);
+          const uint32_t sb = sa + kPlanes * kPA;
+          if (lead) {
 #pragma unroll
             for (int k = 0; k < kPBK / 16; k++) {
               const uint32_t acc = (kb != kb0 || k) ? 1u : 0u;
@@ -255,10 +256,14 @@ pairwise_tc_kernel(const __grid_constant__ PairwiseArgs a, const tc::WaitCfg wc)
             }
             tc::umma_commit(&empty[s]);
           }
-          if (ok) tc::umma_commit(&accf[buf]);
+          __syncwarp();
         }
+        if (ok && lead) tc::umma_commit(&accf[buf]);
+        __syncwarp();
       }
-      if (!ok) *abort_flag = 1;
+    }
+    if (!ok) *abort_flag = 1;
+    if (lead) {
       tc::umma_commit(mma_done);
       tc::mbar_wait_bounded(mma_done, 0u, kPDrainNs);
     }
