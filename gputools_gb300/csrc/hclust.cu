@@ -683,8 +683,9 @@ bool format_clustering(int len, const int *sub, const int *sup, int *merge, int 
 
 // Threads of a CTA: one for each column that it owns, 128 to 512.  More warps cost
 // every step their share of the barriers and reductions (1000 objects, 63 columns
-// a CTA: 128 threads 3.27 ms, 256 3.40, 512 3.9); fewer scan rows slower (4000
-// objects, 250 columns a CTA: 256 threads 14.6 ms, 128 17.2, 512 16.6).
+// a CTA: 128 threads 4.20 ms, 256 4.36, 512 4.79); fewer scan rows slower (4000
+// objects, 250 columns a CTA: 128 threads 21.3 ms, 256 18.1, 512 20.8; both before
+// the step's code was shortened).
 int hc_threads(int64_t n, int G) {
   int t = 128;
   while (t < kHcThreads && t * G < n) t *= 2;
