@@ -29,10 +29,18 @@
 // the epilogue adds each chunk into FP32 running sums and forms r, the t-score
 // and the pair count from them.
 //
+// The operand copies bound the kernel: 50 KB for the 384 tensor-core cycles of a
+// k-block, 130 bytes a cycle where an SM takes in about 45.  Four fifths are the
+// row variables' planes; with BOTH two CTAs of a cluster take neighbouring column
+// tiles of the same rows and each fetches half of those planes for the two, so
+// that L2 gives them out once (1000 observations of 4000 variables 306 -> 290 us,
+// 200 of 4000 126 -> 111).  Tiles that do not fill the SMs run without it (the
+// cluster's start and end: 100 of 300 36.4 -> 38.9).
 // Kernel layout as in gram_tc.cu: persistent, one CTA per SM; warp 0 issues
 // the TMA loads, warp 1 the MMAs, warps 2..17 are the epilogue (4 per TMEM
 // lane quarter, 8 column variables each).  Every mbarrier wait is bounded.
 #include "common.cuh"
+#include "gram_core.cuh"
 #include "kernels.cuh"
 #include "stats.cuh"
 #include "tc_ptx.cuh"
@@ -63,8 +71,8 @@ constexpr uint64_t kPDrainNs = 200000000ull;
 constexpr float kPScale = 16384.f;                 // 2^14
 
 struct PairwiseArgs {
-  CUtensorMap ma, mb;  // 3-D maps over the five planes; boxes of 128 and 32 rows
-  const int2 *tiles;   // (first row variable, first column variable) per tile
+  CUtensorMap ma, mb;  // 3-D maps over the five planes; boxes of 128 (BOTH: 64) and 32 rows
+  const int2 *tiles;   // (first row variable, first column variable) per tile (BOTH: two tiles)
   int64_t ntiles, nk;  // tiles, k-blocks
   float *corr, *ts, *pairs;
   int64_t ld, nr, nc;
@@ -129,11 +137,30 @@ __device__ __forceinline__ void tmem_ld8x2(uint32_t a0, uint32_t a1, float (&v)[
   for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
 
+// From lane = row, v[j] = column j to v[k] = (row 4 k + lane mod 4, column
+// lane / 4): three exchanges of a lane bit with a register bit.
+__device__ __forceinline__ void transpose8(float (&v)[8]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int b = 0; b < 3; b++) {  // register bit b and lane bit b + 2
+    const bool hi = (lane >> (b + 2)) & 1;
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+      if (j & (1 << b)) continue;
+      float &v0 = v[j], &v1 = v[j | (1 << b)];
+      const float got = __shfl_xor_sync(0xffffffffu, hi ? v0 : v1, 4 << b);
+      if (hi) v0 = got;
+      else v1 = got;
+    }
+  }
+}
+
 __device__ __forceinline__ float signif_pw(float r, float pairs) {
   if (r >= 0.999f) return 10000.0f;
   return r * sqrtf((pairs - 2.f) / (1.f - r * r));
 }
 
+template <bool BOTH>
 __global__ void __launch_bounds__(kPThreads, 1)
 pairwise_tc_kernel(const __grid_constant__ PairwiseArgs a, const tc::WaitCfg wc) {
   if (a.run_if && *a.run_if == 0) return;  // a gated launch whose gate is closed
@@ -149,10 +176,12 @@ pairwise_tc_kernel(const __grid_constant__ PairwiseArgs a, const tc::WaitCfg wc)
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = BOTH ? int(tc::cluster_rank()) : 0;
+  const int64_t first = BOTH ? blockIdx.x >> 1 : blockIdx.x, step = BOTH ? gridDim.x >> 1 : gridDim.x;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kPStages; s++) {
       tc::mbar_init(&full[s], 1);
-      tc::mbar_init(&empty[s], 1);
+      tc::mbar_init(&empty[s], BOTH ? 2 : 1);  // every CTA has read the stage
     }
     for (int b = 0; b < 2; b++) {
       tc::mbar_init(&accf[b], 1);
@@ -169,39 +198,50 @@ pairwise_tc_kernel(const __grid_constant__ PairwiseArgs a, const tc::WaitCfg wc)
   if (warp == 1) tc::tmem_alloc(tmem_slot, 512);
   tc::tc_fence_before();
   __syncthreads();
+  if constexpr (BOTH) tc::cluster_sync();  // both CTAs' barriers are there
   tc::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const int64_t nch = (a.nk + kPChunkKb - 1) / kPChunkKb;
 
   if (warp == 0) {
-    if (lane == 0) {
-      // ------------------------------------------------ TMA producer
-      int64_t it = 0;
-      for (int64_t t = blockIdx.x; t < a.ntiles && !*abort_flag; t += gridDim.x) {
-        const int2 tl = a.tiles[t];
-        for (int64_t kb = 0; kb < a.nk; kb++, it++) {
-          const int s = int(it % kPStages);
-          const uint32_t use = uint32_t(it / kPStages);
-          if (!tc::mbar_wait(&empty[s], (use & 1u) ^ 1u, abort_flag, wc)) {
-            *abort_flag = 1;
-            break;
-          }
-          uint8_t *st = smem + s * kPStage;
+    // -------------------------------------------------- TMA producer
+    const int nk = int(a.nk);
+    int it = 0;
+    bool go = true;
+    const bool lead = tc::elect_one();
+    for (int64_t t = first; t < a.ntiles && go && !*abort_flag; t += step) {
+      const int2 tl = a.tiles[t];
+      const int32_t r0 = tl.x + (kPM / 2) * rank, c0 = tl.y + kPN * rank;
+      for (int kb = 0; kb < nk; kb++, it++) {
+        const int s = it % kPStages;
+        go = __all_sync(0xffffffffu, tc::mbar_wait(&empty[s], (uint32_t(it / kPStages) & 1u) ^ 1u,
+                                                   abort_flag, wc));
+        if (!go) {
+          *abort_flag = 1;
+          break;
+        }
+        uint8_t *st = smem + s * kPStage;
+        if (lead) {
           tc::mbar_arrive_expect_tx(&full[s], kPStage);
 #pragma unroll
-          for (int p = 0; p < kPlanes; p++)
-            tc::tma_load_3d(st + p * kPA, &a.ma, &full[s], int32_t(kb * kPBK), tl.x, p);
+          for (int p = 0; p < kPlanes; p++) {
+            uint8_t *dst = st + p * kPA + rank * (kPA / 2);
+            if constexpr (BOTH) tc::tma_load_3d_both(dst, &a.ma, &full[s], kb * kPBK, r0, p);
+            else tc::tma_load_3d(dst, &a.ma, &full[s], kb * kPBK, r0, p);
+          }
 #pragma unroll
           for (int p = 0; p < kPlanes; p++)
-            tc::tma_load_3d(st + kPlanes * kPA + p * kPB, &a.mb, &full[s], int32_t(kb * kPBK),
-                            tl.y, p);
+            tc::tma_load_3d(st + kPlanes * kPA + p * kPB, &a.mb, &full[s], kb * kPBK, c0, p);
         }
+        __syncwarp();
       }
-      if (*abort_flag) {
-        for (int s = 0; s < kPStages; s++) {
-          const int64_t fills = it / kPStages + (s < it % kPStages ? 1 : 0);
-          if (fills > 0) tc::mbar_wait_bounded(&full[s], uint32_t((fills - 1) & 1), kPDrainNs);
-        }
+    }
+    // drain: no bulk copy may still be writing shared memory at exit (with BOTH
+    // time passes below instead)
+    if (!BOTH && *abort_flag && lead) {
+      for (int s = 0; s < kPStages; s++) {
+        const int fills = it / kPStages + (s < it % kPStages ? 1 : 0);
+        if (fills > 0) tc::mbar_wait_bounded(&full[s], uint32_t((fills - 1) & 1), kPDrainNs);
       }
     }
     __syncwarp();
@@ -217,7 +257,7 @@ pairwise_tc_kernel(const __grid_constant__ PairwiseArgs a, const tc::WaitCfg wc)
     int it = 0, cc = 0;
     bool ok = true;
     const bool lead = tc::elect_one();
-    for (int64_t t = blockIdx.x; t < a.ntiles && ok; t += gridDim.x) {
+    for (int64_t t = first; t < a.ntiles && ok; t += step) {
       for (int kb0 = 0; kb0 < nk && ok; kb0 += int(kPChunkKb), cc++) {
         // two accumulator sets: wait until the epilogue has read the set's
         // previous chunk
@@ -254,7 +294,8 @@ pairwise_tc_kernel(const __grid_constant__ PairwiseArgs a, const tc::WaitCfg wc)
               tc::umma_bf16(d + kR4, aqh, b0, id32, acc);
               tc::umma_bf16(d + kR4, aql, b0, id32, 1u);
             }
-            tc::umma_commit(&empty[s]);
+            if constexpr (BOTH) tc::umma_commit_both(&empty[s]);
+            else tc::umma_commit(&empty[s]);
           }
           __syncwarp();
         }
@@ -275,7 +316,7 @@ pairwise_tc_kernel(const __grid_constant__ PairwiseArgs a, const tc::WaitCfg wc)
     const uint32_t lanes = uint32_t(q * 32) << 16;
     int64_t cc = 0;
     bool ok = true;
-    for (int64_t t = blockIdx.x; t < a.ntiles && ok; t += gridDim.x) {
+    for (int64_t t = first; t < a.ntiles && ok; t += step) {
       const int2 tl = a.tiles[t];
       float sN[8], sA[8], sB[8], sAA[8], sBB[8], sAB[8];
 #pragma unroll
@@ -319,13 +360,10 @@ pairwise_tc_kernel(const __grid_constant__ PairwiseArgs a, const tc::WaitCfg wc)
         if (lane == 0) tc::mbar_arrive(&acce[buf]);
       }
       if (!ok) break;
-      const int64_t r = int64_t(tl.x) + q * 32 + lane;
+      const int64_t r = int64_t(tl.x) + q * 32 + lane, c0 = int64_t(tl.y) + rank * kPN + part * 8;
       const float inv = 1.f / kPScale;
 #pragma unroll
-      for (int j = 0; j < 8; j++) {
-        const int64_t c = int64_t(tl.y) + part * 8 + j;
-        if (r >= a.nr || c >= a.nc) continue;
-        if (a.symmetric && r > c) continue;  // the mirror of a computed entry
+      for (int j = 0; j < 8; j++) {  // r into sA, its t-score into sB
         // float from the float sums (the FP64 form gains nothing once they
         // are rounded, and its registers would spill)
         const float N = sN[j];
@@ -341,31 +379,55 @@ pairwise_tc_kernel(const __grid_constant__ PairwiseArgs a, const tc::WaitCfg wc)
             val = rr > 1.f ? 1.f : (rr < -1.f ? -1.f : rr);
           }
         }
-        if (a.symmetric && r == c && val == val) val = 1.f;
-        const float np = N;
-        const float tsv = signif_pw(val, np);
-        const int64_t i0 = r * a.ld + c, i1 = c * a.ld + r;
-        const bool mirror = a.symmetric && r != c;
-        // streaming stores: the outputs, written once, leave the operand
-        // planes in L2
-        if (a.corr) {
-          tc::st_stream(a.corr + i0, val);
-          if (mirror) tc::st_stream(a.corr + i1, val);
-        }
-        if (a.ts) {
-          tc::st_stream(a.ts + i0, tsv);
-          if (mirror) tc::st_stream(a.ts + i1, tsv);
-        }
-        if (a.pairs) {
-          tc::st_stream(a.pairs + i0, np);
-          if (mirror) tc::st_stream(a.pairs + i1, np);
-        }
+        if (a.symmetric && r == c0 + j && val == val) val = 1.f;
+        sA[j] = val;
+        sB[j] = signif_pw(val, N);
       }
+      // Streaming stores: the outputs, written once, leave the operand planes in
+      // L2.  Inside, both orientations as whole sectors: the mirrored rows c from 32
+      // lanes on consecutive columns, rows r after transpose8 (eight columns of
+      // four rows an instruction; one column of 32 rows, an eighth of each
+      // sector, took a third of the kernel's time: 1000 observations of 4000
+      // variables 399 -> 306 us, 200 of 4000 240 -> 126).
+      const int64_t rbase = r - lane;
+      const bool inner = c0 + 8 <= a.nc && rbase + 32 <= a.nr && (!a.symmetric || rbase + 31 < c0);
+      auto put = [&](float *o, float (&v)[8]) {
+        if (!o) return;
+        if (inner) {
+          if (a.symmetric) {
+            float *col = o + c0 * a.ld + r;
+#pragma unroll
+            for (int j = 0; j < 8; j++) tc::st_stream(col + j * a.ld, v[j]);
+          }
+          transpose8(v);
+          float *row = o + (rbase + (lane & 3)) * a.ld + c0 + (lane >> 2);
+#pragma unroll
+          for (int j = 0; j < 8; j++) tc::st_stream(row + 4 * j * a.ld, v[j]);
+        } else if (r < a.nr) {
+#pragma unroll
+          for (int j = 0; j < 8; j++) {
+            const int64_t c = c0 + j;
+            if (c >= a.nc || (a.symmetric && r > c)) continue;  // the mirror of a computed entry
+            tc::st_stream(o + r * a.ld + c, v[j]);
+            if (a.symmetric && r != c) tc::st_stream(o + c * a.ld + r, v[j]);
+          }
+        }
+      };
+      put(a.corr, sA);
+      put(a.ts, sB);
+      put(a.pairs, sN);
     }
     if (!ok) *abort_flag = 1;
   }
   __syncthreads();
-  if (*abort_flag && threadIdx.x == 0) atomicOr(wc.err, 1);
+  if (*abort_flag && threadIdx.x == 0) {
+    atomicOr(wc.err, 1);
+    if (BOTH) tc::pass_time(tc::kCopyTimeNs);  // copies in flight, for both CTAs, end
+  }
+  if constexpr (BOTH) {
+    __syncthreads();
+    tc::cluster_sync();  // the other CTA's copies and commits reach this one's memory
+  }
   if (warp == 1) {
     tc::tc_fence_after();
     tc::tmem_dealloc(tmem_base, 512);
@@ -380,19 +442,26 @@ pairwise_tc_kernel(const __grid_constant__ PairwiseArgs a, const tc::WaitCfg wc)
 int pearson_pairwise_tc(const float *dA, int64_t nA, const float *dB, int64_t nB, int64_t n,
                         const PearsonOut &out, const int *run_if, cudaStream_t s) {
   if (nA == 0 || nB == 0 || n == 0) return GT_OK;
-  if (nA > 2147483647LL - kPM || nB > 2147483647LL - kPN)
+  if (nA > 2147483647LL - kPM || nB > 2147483647LL - 2 * kPN)
     return fail(GT_EINVAL, "too many variables");
   const bool sym = out.symmetric != 0;
   const int64_t kpad = cdiv(n, 64) * 64;
   const size_t bytesA = size_t(kPlanes) * size_t(nA) * size_t(kpad) * 2;
   const size_t bytesB = sym ? 0 : size_t(kPlanes) * size_t(nB) * size_t(kpad) * 2;
-  // tiles: 128 row variables x 32 column variables; for cor(x) those that
-  // reach the upper triangle (column block tj >= 4 ti)
-  const int64_t tr = cdiv(nA, kPM), tcn = cdiv(nB, kPN);
+  // tiles of 128 row variables x 32 column variables, or two of them side by side
+  // where every cluster gets some (see the top); for cor(x) those that reach the
+  // upper triangle
+  const int64_t tr = cdiv(nA, kPM);
   std::vector<int2> tiles;
-  for (int64_t ti = 0; ti < tr; ti++)
-    for (int64_t tj = sym ? 4 * ti : 0; tj < tcn; tj++)
-      tiles.push_back(make_int2(int(ti * kPM), int(tj * kPN)));
+  auto make = [&](int64_t cols) {
+    tiles.clear();
+    for (int64_t ti = 0; ti < tr; ti++)
+      for (int64_t c = sym ? ti * kPM : 0; c < nB; c += cols)
+        tiles.push_back(make_int2(int(ti * kPM), int(c)));
+  };
+  make(2 * kPN);
+  const bool both = 2 * int64_t(tiles.size()) >= sm_count();
+  if (!both) make(kPN);
   if (tiles.empty()) return GT_OK;
   const size_t tbytes = tiles.size() * sizeof(int2);
   void *pw = nullptr;
@@ -412,7 +481,7 @@ int pearson_pairwise_tc(const float *dA, int64_t nA, const float *dB, int64_t nB
     GT_CUDA(cudaGetLastError());
   }
   PairwiseArgs a{};
-  GT_TRY(tc_plane_map(&a.ma, pa, nA, kpad, kPlanes, kPM, kPBK, true));
+  GT_TRY(tc_plane_map(&a.ma, pa, nA, kpad, kPlanes, both ? kPM / 2 : kPM, kPBK, true));
   GT_TRY(tc_plane_map(&a.mb, pb, nB, kpad, kPlanes, kPN, kPBK, true));
   a.tiles = dtiles;
   a.ntiles = int64_t(tiles.size());
@@ -429,11 +498,12 @@ int pearson_pairwise_tc(const float *dA, int64_t nA, const float *dB, int64_t nB
   GT_TRY(device_error_word(&wc.err));
   wc.limit_ns = wait_limit_ns();
   wc.hint_ns = wait_sleep_hint_ns();
-  GT_CUDA(cudaFuncSetAttribute(pairwise_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               kPSmem));
-  const int64_t grid = a.ntiles < sm_count() ? a.ntiles : sm_count();
+  auto kern = both ? pairwise_tc_kernel<true> : pairwise_tc_kernel<false>;
+  GT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPSmem));
   ProfScope prof("pearson_pairwise", s);
-  pairwise_tc_kernel<<<unsigned(grid), kPThreads, kPSmem, s>>>(a, wc);
+  if (both) return launch_pairs(kern, a.ntiles, kPThreads, kPSmem, s, a, wc);
+  const int64_t grid = a.ntiles < sm_count() ? a.ntiles : sm_count();
+  kern<<<unsigned(grid), kPThreads, kPSmem, s>>>(a, wc);
   count_launch();
   GT_CUDA(cudaGetLastError());
   return GT_OK;
