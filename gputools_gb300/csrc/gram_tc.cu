@@ -699,16 +699,16 @@ using FinOf = std::decay_t<decltype(std::declval<const Work &>().finish(std::dec
 
 // One contraction whose K range is cut into `parts` pieces, so that a
 // contraction of few output tiles still occupies the SMs: work item u is
-// output tile u / parts over the k-blocks of piece u % parts, stored by
-// fins[piece] (each piece into its own partial output).
-template <class Fin>
+// output tile u / parts over the k-blocks of piece u % parts, stored into the
+// piece's own partial output (part_stride floats apart).
 struct KSplitWork {
-  static constexpr int kMaxParts = 4;
   CUtensorMap ma, mb;
   TileSpace ts;
   int64_t nk_total, nk_part;
   int parts;
-  Fin fins[kMaxParts];
+  int64_t part_stride;
+  StoreFinish fin;
+  const int *gate = nullptr;  // when set, the kernel does nothing unless *gate == 0
   __device__ bool tile(int64_t cursor, TileRef &ref) const {
     const int64_t u = int64_t(blockIdx.x) + cursor * int64_t(gridDim.x);
     if (u >= ts.ntiles * parts) return false;
@@ -726,9 +726,13 @@ struct KSplitWork {
     return true;
   }
   static constexpr bool kPrefetch = false;
-  __device__ bool skip() const { return false; }
-  __device__ const Fin &finish(const TileRef &ref) const { return fins[ref.prob]; }
-  __device__ void drain(EpiCtx &ctx) const { fins[0].drain(ctx); }
+  __device__ bool skip() const { return gate && *gate != 0; }
+  __device__ StoreFinish finish(const TileRef &ref) const {
+    StoreFinish f = fin;
+    f.out += ref.prob * part_stride;
+    return f;
+  }
+  __device__ void drain(EpiCtx &ctx) const { fin.drain(ctx); }
   __device__ void prefetch() const {
     tc::prefetch_tensormap(&ma);
     tc::prefetch_tensormap(&mb);
@@ -1555,21 +1559,20 @@ int gemm_tc_store_ksplit(const void *planesA, int64_t nA, const void *planesB, i
                          cudaStream_t s) {
   *used = 0;
   if (nA == 0 || nB == 0) return GT_OK;
-  using W = KSplitWork<StoreFinish>;
   constexpr int BK = 32;
   if (kpad <= 0 || kpad % BK) return fail(GT_EINVAL, "bad padded K (%lld)", (long long)kpad);
   const int64_t nk = kpad / BK;
-  if (parts < 1 || parts > W::kMaxParts) return fail(GT_EINVAL, "bad K split (%d)", parts);
+  if (parts < 1 || parts > 4) return fail(GT_EINVAL, "bad K split (%d)", parts);
   if (parts > nk) parts = int(nk);
-  W w;
+  KSplitWork w;
   GT_TRY(make_plane_map(&w.ma, planesA, nA, kpad, 3, kBM, BK, false));
   GT_TRY(make_plane_map(&w.mb, planesB, nB, kpad, 3, kBN, BK, false));
   w.ts = make_tiles(nA, nB, kFull, band_group(int64_t(kBN) * kpad * 2 * 3));
   w.nk_total = nk;
   w.nk_part = cdiv(nk, int64_t(parts));
   w.parts = int(cdiv(nk, w.nk_part));  // every piece non-empty
-  for (int q = 0; q < w.parts; q++)
-    w.fins[q] = StoreFinish{C + int64_t(q) * nA * ldc, ldc, nA, nB};
+  w.part_stride = nA * ldc;
+  w.fin = StoreFinish{C, ldc, nA, nB};
   *used = w.parts;
   return launch_work<tc::KIND_BF16X6, BK, true>(w, w.ts.ntiles * w.parts, tc_chunk_kblocks(BK),
                                                 "gemm_store", s);
@@ -1585,6 +1588,87 @@ int gemm_tc_store_scaled(const void *planesA, int64_t nA, const void *planesB, i
   return launch_gram<tc::KIND_F16X3, 32, true>(planesA, nA, planesB, nB, kpad, kFull,
                                                tc_chunk_kblocks(32), fin, "gemm_store", s);
 }
+
+namespace {
+
+// The Pearson outputs from the pieces of a split contraction (P: [piece][nr][nc]):
+// 32 x 32 entries a block, the mirror entries through its tile.
+__global__ void __launch_bounds__(256)
+pearson_parts_kernel(const PearsonFinish fin, const float *__restrict__ P, int parts) {
+  __shared__ float tile[32][33];
+  if (fin.skip()) return;
+  const int64_t c0 = int64_t(blockIdx.x) * 32, r0 = int64_t(blockIdx.y) * 32;
+  if (!fin.block_live(r0, c0)) return;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int64_t c = c0 + tx, piece = fin.nr * fin.nc;
+  float v[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 2
+  for (int q = 0; q < parts; q++) {
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const int64_t r = r0 + ty + 8 * k;
+      if (r < fin.nr && c < fin.nc) v[k] += P[q * piece + r * fin.nc + c];
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const int64_t r = r0 + ty + 8 * k, o = r * fin.ld + c;
+    float x = clamp_r(v[k] * fin.gscale);
+    tile[ty + 8 * k][tx] = x;
+    if (r >= fin.nr || c >= fin.nc || (fin.symmetric && r > c)) continue;
+    if (fin.symmetric && r == c && x == x) x = 1.f;
+    fin.put(fin.corr + o, fin.ts + o, fin.pairs + o, x);
+  }
+  if (!fin.symmetric) return;
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const int64_t r = r0 + tx, cc = c0 + ty + 8 * k, o = cc * fin.ld + r;
+    if (cc >= fin.nc || r >= cc) continue;
+    fin.put(fin.corr + o, fin.ts + o, fin.pairs + o, tile[tx][ty + 8 * k]);
+  }
+}
+
+// The f16x3 Pearson Gram of few tiles with its observations cut into pieces, as many
+// as give every SM one, up to 16 of at least 128 observations: true if taken (a
+// tile's k-blocks are a serial chain, about half a microsecond each, on a few
+// SMs).  Measured, whole / in pieces: 4096 observations of 700 variables 94 / 40
+// us, of 1700 105 / 78, 2000 of 1200 64 / 39, 1000 of 1000 47 / 30, 500 of 1200
+// 39 / 31 (pieces of at least 256: 33, 512: 39), 4096 of 200 x 2000 109 / 70.
+bool pearson_split(const void *zA, int64_t nA, const void *zB, int64_t nB, int64_t kpad, int sym,
+                   const PearsonFinish &fin, cudaStream_t s, int *status) {
+  constexpr int BK = 32;
+  KSplitWork w;
+  w.ts = make_tiles(nA, nB, sym, band_group(int64_t(kBN) * kpad * 2 * 2));
+  const int64_t nk = kpad / BK;
+  const int64_t want = std::min<int64_t>(sm_count() / w.ts.ntiles, std::min<int64_t>(nk / 4, 16));
+  if (want < 2) return false;
+  w.nk_total = nk;
+  w.nk_part = cdiv(nk, want);
+  w.parts = int(cdiv(nk, w.nk_part));
+  void *P = nullptr;
+  if (ws_get(WS_ADJ1, size_t(w.parts) * size_t(nA) * size_t(nB) * 4, &P) != GT_OK) {
+    clear_error();  // no room for the pieces: in one
+    return false;
+  }
+  w.part_stride = nA * nB;
+  w.fin = StoreFinish{static_cast<float *>(P), nB, nA, nB};
+  w.gate = fin.gate;
+  *status = [&]() -> int {
+    GT_TRY(make_plane_map(&w.ma, zA, nA, kpad, 2, kBM, BK, true));
+    GT_TRY(make_plane_map(&w.mb, zB, nB, kpad, 2, kBN, BK, true));
+    GT_TRY((launch_work<tc::KIND_F16X3, BK, true>(w, w.ts.ntiles * w.parts, tc_chunk_kblocks(BK),
+                                                  "pearson_gram", s)));
+    pearson_parts_kernel<<<dim3(unsigned(cdiv(nB, 32)), unsigned(cdiv(nA, 32))), 256, 0, s>>>(
+        fin, static_cast<const float *>(P), w.parts);
+    count_launch();
+    GT_CUDA(cudaGetLastError());
+    return GT_OK;
+  }();
+  return true;
+}
+
+}  // namespace
 
 int pearson_tc_prologue(const float *dX, int64_t nvar, int64_t n, int kind, int slot_z,
                         int slot_st, void **Z, int64_t *kpad, cudaStream_t s,
@@ -1631,6 +1715,9 @@ int pearson_tc(const void *zA, int64_t nA, const void *zB, int64_t nB, int64_t k
     return launch_gram<tc::KIND_BF16X6, 32, true>(zA, nA, zB, nB, kpad, sym, tc_chunk_kblocks(32),
                                                   fin, "pearson_gram", s);
   if (kind == tc::KIND_F16X3) {
+    int status = GT_OK;
+    if (tc_config() == 32 && pearson_split(zA, nA, zB, nB, kpad, sym, fin, s, &status))
+      return status;
     if (tc_config() == 32)
       return launch_gram<tc::KIND_F16X3, 32, true>(zA, nA, zB, nB, kpad, sym,
                                                    tc_chunk_kblocks(32), fin, "pearson_gram", s);

@@ -158,15 +158,17 @@ pearson_fma_kernel(const float *__restrict__ ZA, const float *__restrict__ ZB, i
 
 }  // namespace
 
-// Whether pearson_fma takes the problem.  Measured against the tensor-core Gram
-// (us a call, here / there): 40 obs x 100 variables 23 / 35 (23 is the host's
-// share), 500 x 200 24 / 43, 500 x 1000 34 / 44, 1000 x 700 43 / 53, 2000 x 500
-// 58 / 72, 4000 x 60 78 / 98, 100 x 1500 26 / 37, 1000 obs x 4000 and 20 variables
-// 34 / 49; past the limits 500 x 2000 89 / 47 and 100 x 2000 38 / 37 (outputs).
+// Whether pearson_fma takes the problem.  Measured against the tensor-core Gram with
+// its observations in pieces (us a call, here / there): 40 obs x 100 variables 23 /
+// 31 (23 is the host's share), 700 x 400 25 / 32, 1000 x 300 23 / 31, 1500 x 250 31 /
+// 31, 250 x 900 23 / 31, 100 x 1500 27 / 31, 2000 obs x 200 and 500 variables 37 / 43,
+// 1500 x 20 and 4000 42 / 44; past the limits 1000 x 500 33 / 30, 400 x 1000 31 / 29,
+// 4000 x 200 73 / 37 (a tile walks all observations), 100 x 1700 33 / 31 (outputs),
+// 2500 x 50 and 2000 55 / 49.
 // The relative error of r falls from 1.2e-7 .. 1.1e-6 to 0.2e-7 .. 1.5e-7.
 bool pearson_fma_wins(int64_t nA, int64_t nB, int64_t n, int symmetric) {
   const double entries = double(nA) * double(nB);
-  return n <= 4096 && entries <= 3e6 && entries * double(n) <= (symmetric ? 5e8 : 2.5e8);
+  return n <= (symmetric ? 1500 : 2000) && entries <= 2.5e6 && entries * double(n) <= 2.4e8;
 }
 
 int pearson_fma(const float *dA, int64_t nA, const float *dB, int64_t nB, int64_t n,
