@@ -141,12 +141,10 @@ constexpr int simt_min_blocks() { return TM * TN * NACC <= 64 ? 2 : 1; }
 // Writes a tile's entries (and mirror) from the accumulators; T is the operand
 // buffer, idle by now (every thread has passed the main loop's last barrier).
 template <class Out, int TM, int TN, int NA>
-__device__ __forceinline__ void simt_write_tile(const SimtArgs &a, const Out &out, int ti, int tj,
-                                                int64_t row0, int64_t col0, float *T,
-                                                float (&acc)[TM][TN][NA]) {
+__device__ __forceinline__ void simt_write_tile(const SimtArgs &a, const Out &out, bool mirror,
+                                                int tx, int ty, int64_t row0, int64_t col0,
+                                                float *T, float (&acc)[TM][TN][NA]) {
   constexpr int BM = 16 * TM, BN = 16 * TN, LDA = simt_ld<BM>();
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const bool mirror = a.symmetric && ti != tj;
   if constexpr (HasStagedMirror<Out>::value) {
     if (out.staged(mirror)) {
       // the tile's entries, then its mirror in 32-row chunks through the
@@ -273,7 +271,8 @@ allpairs_simt_kernel(SimtArgs a, Op op, Out out) {
     __syncthreads();
   }
 
-  simt_write_tile<Out, TM, TN, NA>(a, out, ti, tj, row0, col0, &sA[0][0], acc);
+  simt_write_tile<Out, TM, TN, NA>(a, out, a.symmetric && ti != tj, tx, ty, row0, col0, &sA[0][0],
+                                   acc);
 }
 
 template <class Op, class Out, int TM, int TN>

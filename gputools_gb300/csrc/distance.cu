@@ -388,7 +388,8 @@ canberra_kernel(SimtArgs a, const unsigned *__restrict__ bits, int64_t words,
     for (int j = 0; j < TN; j++)
       val[i][j][0] = canberra_finish(j & 1 ? acc[i][j / 2].y : acc[i][j / 2].x,
                                      int(a.K - used[i][j]), a.K);
-  simt_write_tile<OutDist<OpValue>, TM, TN, 1>(a, out, ti, tj, row0, col0, &sA[0][0], val);
+  simt_write_tile<OutDist<OpValue>, TM, TN, 1>(a, out, a.symmetric && ti != tj, tx, ty, row0, col0,
+                                               &sA[0][0], val);
 }
 
 SimtArgs dist_args(const float *pts, int64_t n, int64_t dim) {
