@@ -220,7 +220,7 @@ int any_nan_flag(const float *a, int64_t na, const float *b, int64_t nb, int **f
 
 }  // namespace
 
-// Column statistics (FP64 mean, inverse norm, flags) of nvar variables.
+// Column statistics (mean and inverse norm as float pairs, flags) of nvar variables.
 int launch_colstats(const float *dX, int64_t nvar, int64_t n, int use, ColStats *st,
                     cudaStream_t s) {
   if (nvar == 0) return GT_OK;
