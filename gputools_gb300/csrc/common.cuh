@@ -58,10 +58,10 @@ enum WsSlot {
   WS_IN_A = 0, WS_IN_B, WS_OUT0, WS_OUT1, WS_OUT2, WS_SCRATCH0, WS_SCRATCH1,
   WS_SCRATCH2, WS_SCRATCH3, WS_SCRATCH4,
   // the distance adjoint's own slots (it calls the Euclid path, which uses
-  // WS_SCRATCH0..3, in between); WS_ADJ1 also holds the pieces of a split
-  // Pearson Gram
+  // WS_SCRATCH0..3, in between)
   WS_ADJ0, WS_ADJ1, WS_ADJ2,
   WS_TILES,  // tile tables of banded launches
+  WS_PARTS,  // the pieces of a split Pearson Gram
   WS_NSLOTS
 };
 // Device buffer of at least `bytes` for `slot` on the current device.

@@ -1402,11 +1402,15 @@ int launch_gram(const void *zA, int64_t nA, const void *zB, int64_t nB, int64_t 
     // SMs idle that 128 x 256 ones would use).  f16x3, single CTAs against pairs:
     // 500 observations x 2817 variables (78 tiles) 74 -> 57 us, x 10000 270 -> 263,
     // 4096 x 20000 3766 -> 3587, mutual information of 1000 x 2000 (10 bins) 703 ->
-    // 664; where the outputs bound it, 100 x 12000, 304 -> 310.
+    // 664; where the outputs bound it, 100 x 12000, 304 -> 310.  From 1024 observations
+    // four fifths of the pairs are enough: 2000 of 2000 x 2000 (64 tiles) 80 -> 77.5,
+    // the adjoint of 1024 x 4096 154 -> 151.5; 500 of 2000 x 2000 37 -> 39.
     const PairSpace ps = make_pair_space(nA, nB, mode == kUpper ? 1 : 0,
                                          band_group(int64_t(kBN) * kpad * tc::Kind<KIND>::NSPLIT));
-    if (2 * ps.ntiles >= sm_count() && ps.ntiles <= 2147483647LL && nA > kBM && mode != kLower &&
-        kpad > 0 && kpad % kKPad == 0) {
+    const bool enough = 2 * ps.ntiles >= sm_count() ||
+                        (kpad >= 1024 && 5 * ps.ntiles >= 2 * int64_t(sm_count()));
+    if (enough && ps.ntiles <= 2147483647LL && nA > kBM && mode != kLower && kpad > 0 &&
+        kpad % kKPad == 0) {
       using PC = TcCfg<KIND, BK, false, false, true>;
       PairWork<Fin> w;
       GT_TRY(make_plane_map(&w.ma, zA, nA, kpad, PC::NSPLIT, kBM, BK, tc::Kind<KIND>::F16));
@@ -1647,7 +1651,7 @@ bool pearson_split(const void *zA, int64_t nA, const void *zB, int64_t nB, int64
   w.nk_part = cdiv(nk, want);
   w.parts = int(cdiv(nk, w.nk_part));
   void *P = nullptr;
-  if (ws_get(WS_ADJ1, size_t(w.parts) * size_t(nA) * size_t(nB) * 4, &P) != GT_OK) {
+  if (ws_get(WS_PARTS, size_t(w.parts) * size_t(nA) * size_t(nB) * 4, &P) != GT_OK) {
     clear_error();  // no room for the pieces: in one
     return false;
   }
