@@ -438,6 +438,105 @@ struct PearsonFinish {
   __device__ void drain(EpiCtx &) const {}
 };
 
+// Plain FP32 store of the contraction, C[r*ld + c]; with row and column
+// scales (operands scaled per row by powers of two), C[r][c] * rs[r] * cs[c].
+struct StoreFinish {
+  float *out;
+  int64_t ld, nr, nc;
+  const float *rs = nullptr, *cs = nullptr;
+  __device__ void operator()(int64_t r, int64_t c0, const float (&g)[32], EpiCtx &ctx) const {
+    const int lane = threadIdx.x & 31;
+    float *wsm = ctx.wsm;
+#pragma unroll
+    for (int j = 0; j < 32; j++) wsm[lane * 33 + j] = g[j];
+    __syncwarp();
+    const int64_t rbase = r - lane, c = c0 + lane;
+    const float csc = (rs && c < nc) ? cs[c] : 1.f;
+    if (rbase + 31 < nr && c0 + 31 < nc) {
+      float *o = out + (rbase * ld + c);
+      if (rs) {
+#pragma unroll 8
+        for (int i = 0; i < 32; i++) {
+          *o = (wsm[i * 33 + lane] * rs[rbase + i]) * csc;
+          o += ld;
+        }
+      } else {
+#pragma unroll 8
+        for (int i = 0; i < 32; i++) {
+          *o = wsm[i * 33 + lane];
+          o += ld;
+        }
+      }
+      __syncwarp();
+      return;
+    }
+    for (int i = 0; i < 32; i++) {
+      const int64_t ri = rbase + i;
+      if (ri >= nr) break;
+      if (c < nc) out[ri * ld + c] = rs ? (wsm[i * 33 + lane] * rs[ri]) * csc : wsm[i * 33 + lane];
+    }
+    __syncwarp();
+  }
+  __device__ void begin_tile(int64_t, EpiCtx &) const {}
+  __device__ void end_tile(EpiCtx &) const {}
+  __device__ void drain(EpiCtx &) const {}
+};
+
+// The Pearson outputs from the pieces of a split contraction: P holds parts x SUMS
+// matrices nr x nc (SUMS 3: the sums S0, S1, S2 of the error-free Gram).  32 x 32
+// entries a block, the mirror entries through its tile.
+template <int SUMS>
+__global__ void __launch_bounds__(256)
+pearson_parts_kernel(const PearsonFinish fin, const float *__restrict__ P, int parts) {
+  __shared__ float tile[32][33];
+  if (fin.skip()) return;
+  const int64_t c0 = int64_t(blockIdx.x) * 32, r0 = int64_t(blockIdx.y) * 32;
+  if (!fin.block_live(r0, c0)) return;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int64_t c = c0 + tx, piece = fin.nr * fin.nc;
+  float v[SUMS][4] = {};
+#pragma unroll 2
+  for (int q = 0; q < parts; q++) {
+#pragma unroll
+    for (int s = 0; s < SUMS; s++) {
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        const int64_t r = r0 + ty + 8 * k;
+        if (r < fin.nr && c < fin.nc) v[s][k] += P[(q * SUMS + s) * piece + r * fin.nc + c];
+      }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    float g = v[0][k];
+    if constexpr (SUMS == 3)  // 2^-24 S2 + 2^-12 S1 + S0
+      g += fmaf(v[1][k], 2.44140625e-4f, v[2][k] * 5.9604644775390625e-8f);
+    const int64_t r = r0 + ty + 8 * k, o = r * fin.ld + c;
+    float x = clamp_r(g * fin.gscale);
+    tile[ty + 8 * k][tx] = x;
+    if (r >= fin.nr || c >= fin.nc || (fin.symmetric && r > c)) continue;
+    if (fin.symmetric && r == c && x == x) x = 1.f;
+    fin.put(fin.corr + o, fin.ts + o, fin.pairs + o, x);
+  }
+  if (!fin.symmetric) return;
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const int64_t r = r0 + tx, cc = c0 + ty + 8 * k, o = cc * fin.ld + r;
+    if (cc >= fin.nc || r >= cc) continue;
+    fin.put(fin.corr + o, fin.ts + o, fin.pairs + o, tile[tx][ty + 8 * k]);
+  }
+}
+
+// Pieces of a contraction of nk 32-wide k-blocks over `tiles` tiles: as many as give
+// every SM one, up to 16 of at least `least` k-blocks (1: in one).
+inline int k_pieces(int64_t tiles, int64_t nk, int64_t least) {
+  int64_t want = sm_count() / (tiles > 0 ? tiles : 1);
+  if (want > nk / least) want = nk / least;
+  if (want > 16) want = 16;
+  return want < 2 ? 1 : int(cdiv(nk, cdiv(nk, want)));  // every piece non-empty
+}
+
 // ----------------------------------------------------------------- work sources
 // A work source tells every role of the kernel, for the cursor-th tile of
 // this CTA, which tensor maps to load from, the tile's row / column blocks,

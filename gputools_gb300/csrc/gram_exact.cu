@@ -103,6 +103,40 @@ __device__ __forceinline__ bool half_live(const PearsonFinish &fin, const TileRe
   return true;
 }
 
+// A problem with its k-blocks in pieces (work item u: tile u / parts, piece u %
+// parts), whose three sums are stored, not finished: S0 and S1 of the pieces add
+// exactly in FP32, as they do in the accumulators.
+struct ExactPieces {
+  CUtensorMap ma, mb;
+  TileSpace ts;
+  int64_t nk_total, nk_part;
+  int parts;
+  PearsonFinish fin;
+  float *out;  // [piece][sum][nr][nc]
+  __device__ bool tile(int64_t cursor, TileRef &ref) const {
+    const int64_t u = int64_t(blockIdx.x) + cursor * int64_t(gridDim.x);
+    if (u >= ts.ntiles * parts) return false;
+    const int64_t t = u / parts, piece = u - t * parts;
+    int64_t ti, tj;
+    tile_coords(ts, t, ti, tj);
+    ref.row0 = ti * kBM;
+    ref.col0 = tj * kBN;
+    ref.ma = &ma;
+    ref.mb = &mb;
+    ref.k0 = piece * nk_part;
+    ref.nk = nk_total - ref.k0 < nk_part ? nk_total - ref.k0 : nk_part;
+    ref.prob = piece;
+    return true;
+  }
+  static constexpr bool kPrefetch = false;
+  __device__ bool skip() const { return fin.skip(); }
+  __device__ const PearsonFinish &finish(const TileRef &) const { return fin; }
+  __device__ void prefetch() const {
+    tc::prefetch_tensormap(&ma);
+    tc::prefetch_tensormap(&mb);
+  }
+};
+
 template <class Work, bool PAIR>
 __global__ void __launch_bounds__(kXThreads, 1)
 gram_exact_kernel(const __grid_constant__ Work work, const tc::WaitCfg wc) {
@@ -152,7 +186,7 @@ gram_exact_kernel(const __grid_constant__ Work work, const tc::WaitCfg wc) {
     bool go = true;
     while (go && !*abort_flag && tiles.next(ref)) {
       const auto &fin = work.finish(ref);
-      const int nk = int(ref.nk);
+      const int nk = int(ref.nk), k0 = int(ref.k0);
       for (int h = 0; h < 2 && go; h++) {
         if (!half_live(fin, ref, h)) continue;
         const int32_t r0 = int32_t(ref.row0) + rank * kBM;
@@ -171,9 +205,9 @@ gram_exact_kernel(const __grid_constant__ Work work, const tc::WaitCfg wc) {
             if (rank == 0) tc::mbar_arrive_expect_tx(&full[s], (PAIR ? 2 : 1) * kXStage);
             auto load = [&](void *dst, const CUtensorMap *map, int32_t row, int p) {
               if constexpr (PAIR)
-                tc::tma_load_3d_pair(dst, map, &full[s], kb * kXBK, row, p);
+                tc::tma_load_3d_pair(dst, map, &full[s], (k0 + kb) * kXBK, row, p);
               else
-                tc::tma_load_3d(dst, map, &full[s], kb * kXBK, row, p);
+                tc::tma_load_3d(dst, map, &full[s], (k0 + kb) * kXBK, row, p);
             };
 #pragma unroll
             for (int p = 0; p < kXPlanes; p++) load(st + p * kXATile, ref.ma, r0, p);
@@ -290,31 +324,47 @@ gram_exact_kernel(const __grid_constant__ Work work, const tc::WaitCfg wc) {
         }
         tc::tc_fence_after();
         const uint32_t tb = tmem_base + uint32_t(part * kXCols) + (uint32_t(q * 32) << 16);
-        float g[2][32];
+        if constexpr (std::is_same<Work, ExactPieces>::value) {
+#pragma unroll 1
+          for (int a = 0; a < 6; a++) {  // sum a / 2, columns 32 (a mod 2) ..
+            float t[32];
+            tc::tmem_ld32(tb + uint32_t((a >> 1) * kXB + 32 * (a & 1)), t);
+            const StoreFinish st{work.out + (ref.prob * 3 + (a >> 1)) * fin.nr * fin.nc, fin.nc, fin.nr,
+                                 fin.nc};
+            st(r, col + 32 * (a & 1), t, ctx);
+            __syncwarp();
+          }
+          tc::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) tc::mbar_arrive(acce);
+          hc++;
+        } else {
+          float g[2][32];
 #pragma unroll
-        for (int i = 0; i < 2; i++) {
-          float t[32];
-          tc::tmem_ld32(tb + uint32_t(2 * kXB + 32 * i), t);  // S2
+          for (int i = 0; i < 2; i++) {
+            float t[32];
+            tc::tmem_ld32(tb + uint32_t(2 * kXB + 32 * i), t);  // S2
 #pragma unroll
-          for (int j = 0; j < 32; j++) g[i][j] = t[j] * 5.9604644775390625e-8f;  // 2^-24
-          tc::tmem_ld32(tb + uint32_t(kXB + 32 * i), t);  // S1
+            for (int j = 0; j < 32; j++) g[i][j] = t[j] * 5.9604644775390625e-8f;  // 2^-24
+            tc::tmem_ld32(tb + uint32_t(kXB + 32 * i), t);  // S1
 #pragma unroll
-          for (int j = 0; j < 32; j++) g[i][j] = fmaf(t[j], 2.44140625e-4f, g[i][j]);  // 2^-12
-          tc::tmem_ld32(tb + uint32_t(32 * i), t);  // S0
+            for (int j = 0; j < 32; j++) g[i][j] = fmaf(t[j], 2.44140625e-4f, g[i][j]);  // 2^-12
+            tc::tmem_ld32(tb + uint32_t(32 * i), t);  // S0
 #pragma unroll
-          for (int j = 0; j < 32; j++) g[i][j] += t[j];
+            for (int j = 0; j < 32; j++) g[i][j] += t[j];
+          }
+          tc::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) {
+            if constexpr (PAIR) tc::mbar_arrive_cta(acce, 0);
+            else tc::mbar_arrive(acce);
+          }
+          hc++;
+          fin.begin_tile(r, ctx);
+          fin(r, col, g[0], ctx);
+          fin(r, col + 32, g[1], ctx);
+          fin.end_tile(ctx);
         }
-        tc::tc_fence_before();
-        __syncwarp();
-        if (lane == 0) {
-          if constexpr (PAIR) tc::mbar_arrive_cta(acce, 0);
-          else tc::mbar_arrive(acce);
-        }
-        hc++;
-        fin.begin_tile(r, ctx);
-        fin(r, col, g[0], ctx);
-        fin(r, col + 32, g[1], ctx);
-        fin.end_tile(ctx);
       }
     }
     if (!ok) *abort_flag = 1;
@@ -520,12 +570,40 @@ int pearson_exact(const void *zA, int64_t nA, const void *zB, int64_t nB, int64_
     w.fin = exact_finish(out, nA, nB);
     return launch_exact_pair(w, s);
   }
+  const int mode = out.symmetric ? kUpper : kFull;
+  const TileSpace ts = make_tiles(nA, nB, mode, band_group(panel));
+  // Few tiles: the observations in pieces of at least 512 (a tile's k-blocks are a
+  // serial chain on one SM).  Whole / in pieces (us): 4096 of 700 variables 178 /
+  // 74, of 1700 193 / 142, of 200 x 2000 210 / 117, 2000 of 1200 100 / 66, of 100 63 /
+  // 39, 1000 of 1000 63 / 53.  Pieces of 256 help at 1000 (48) and cost at 500 of
+  // 2000 variables (43 / 54: three matrices a piece are written and read).
+  const int pieces = k_pieces(ts.ntiles, kpad / kXBK, 16);
+  void *P = nullptr;
+  if (pieces > 1) {
+    if (ws_get(WS_PARTS, size_t(pieces) * 3 * size_t(nA) * size_t(nB) * 4, &P) == GT_OK) {
+      ExactPieces w;
+      GT_TRY(tc_plane_map(&w.ma, zA, nA, kpad, kXPlanes, kBM, kXBK, true));
+      GT_TRY(tc_plane_map(&w.mb, zB, nB, kpad, kXPlanes, kXB, kXBK, true));
+      w.ts = ts;
+      w.nk_total = kpad / kXBK;
+      w.nk_part = cdiv(w.nk_total, int64_t(pieces));
+      w.parts = pieces;
+      w.fin = exact_finish(out, nA, nB);
+      w.out = static_cast<float *>(P);
+      GT_TRY(launch_exact(w, ts.ntiles * pieces, s));
+      pearson_parts_kernel<3><<<dim3(unsigned(cdiv(nB, 32)), unsigned(cdiv(nA, 32))), 256, 0, s>>>(
+          w.fin, w.out, pieces);
+      count_launch();
+      GT_CUDA(cudaGetLastError());
+      return GT_OK;
+    }
+    clear_error();  // no room for the pieces: in one
+  }
   using W = SingleWork<PearsonFinish>;
   W w;
   GT_TRY(tc_plane_map(&w.ma, zA, nA, kpad, kXPlanes, kBM, kXBK, true));
   GT_TRY(tc_plane_map(&w.mb, zB, nB, kpad, kXPlanes, kXB, kXBK, true));
-  const int mode = out.symmetric ? kUpper : kFull;
-  w.ts = make_tiles(nA, nB, mode, band_group(panel));
+  w.ts = ts;
   if (w.ts.ntiles > 2147483647LL)
     return fail(GT_EINVAL, "problem too large (%lld tiles)", (long long)w.ts.ntiles);
   w.nk = kpad / kXBK;

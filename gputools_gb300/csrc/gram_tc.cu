@@ -567,50 +567,6 @@ struct MiFinish {
   __device__ void drain(EpiCtx &) const {}
 };
 
-// Plain FP32 store of the contraction, C[r*ld + c]; with row and column
-// scales (operands scaled per row by powers of two), C[r][c] * rs[r] * cs[c].
-struct StoreFinish {
-  float *out;
-  int64_t ld, nr, nc;
-  const float *rs = nullptr, *cs = nullptr;
-  __device__ void operator()(int64_t r, int64_t c0, const float (&g)[32], EpiCtx &ctx) const {
-    const int lane = threadIdx.x & 31;
-    float *wsm = ctx.wsm;
-#pragma unroll
-    for (int j = 0; j < 32; j++) wsm[lane * 33 + j] = g[j];
-    __syncwarp();
-    const int64_t rbase = r - lane, c = c0 + lane;
-    const float csc = (rs && c < nc) ? cs[c] : 1.f;
-    if (rbase + 31 < nr && c0 + 31 < nc) {
-      float *o = out + (rbase * ld + c);
-      if (rs) {
-#pragma unroll 8
-        for (int i = 0; i < 32; i++) {
-          *o = (wsm[i * 33 + lane] * rs[rbase + i]) * csc;
-          o += ld;
-        }
-      } else {
-#pragma unroll 8
-        for (int i = 0; i < 32; i++) {
-          *o = wsm[i * 33 + lane];
-          o += ld;
-        }
-      }
-      __syncwarp();
-      return;
-    }
-    for (int i = 0; i < 32; i++) {
-      const int64_t ri = rbase + i;
-      if (ri >= nr) break;
-      if (c < nc) out[ri * ld + c] = rs ? (wsm[i * 33 + lane] * rs[ri]) * csc : wsm[i * 33 + lane];
-    }
-    __syncwarp();
-  }
-  __device__ void begin_tile(int64_t, EpiCtx &) const {}
-  __device__ void end_tile(EpiCtx &) const {}
-  __device__ void drain(EpiCtx &) const {}
-};
-
 // ----------------------------------------------------------------- kernel
 // LISTS: the unchunked (Euclidean) kernel, whose epilogue is latency-bound:
 // 16 epilogue warps of 64 columns, each with a pending-pair list and its
@@ -1595,44 +1551,6 @@ int gemm_tc_store_scaled(const void *planesA, int64_t nA, const void *planesB, i
 
 namespace {
 
-// The Pearson outputs from the pieces of a split contraction (P: [piece][nr][nc]):
-// 32 x 32 entries a block, the mirror entries through its tile.
-__global__ void __launch_bounds__(256)
-pearson_parts_kernel(const PearsonFinish fin, const float *__restrict__ P, int parts) {
-  __shared__ float tile[32][33];
-  if (fin.skip()) return;
-  const int64_t c0 = int64_t(blockIdx.x) * 32, r0 = int64_t(blockIdx.y) * 32;
-  if (!fin.block_live(r0, c0)) return;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int64_t c = c0 + tx, piece = fin.nr * fin.nc;
-  float v[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 2
-  for (int q = 0; q < parts; q++) {
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const int64_t r = r0 + ty + 8 * k;
-      if (r < fin.nr && c < fin.nc) v[k] += P[q * piece + r * fin.nc + c];
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const int64_t r = r0 + ty + 8 * k, o = r * fin.ld + c;
-    float x = clamp_r(v[k] * fin.gscale);
-    tile[ty + 8 * k][tx] = x;
-    if (r >= fin.nr || c >= fin.nc || (fin.symmetric && r > c)) continue;
-    if (fin.symmetric && r == c && x == x) x = 1.f;
-    fin.put(fin.corr + o, fin.ts + o, fin.pairs + o, x);
-  }
-  if (!fin.symmetric) return;
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const int64_t r = r0 + tx, cc = c0 + ty + 8 * k, o = cc * fin.ld + r;
-    if (cc >= fin.nc || r >= cc) continue;
-    fin.put(fin.corr + o, fin.ts + o, fin.pairs + o, tile[tx][ty + 8 * k]);
-  }
-}
-
 // The f16x3 Pearson Gram of few tiles with its observations cut into pieces, as many
 // as give every SM one, up to 16 of at least 128 observations: true if taken (a
 // tile's k-blocks are a serial chain, about half a microsecond each, on a few
@@ -1645,11 +1563,10 @@ bool pearson_split(const void *zA, int64_t nA, const void *zB, int64_t nB, int64
   KSplitWork w;
   w.ts = make_tiles(nA, nB, sym, band_group(int64_t(kBN) * kpad * 2 * 2));
   const int64_t nk = kpad / BK;
-  const int64_t want = std::min<int64_t>(sm_count() / w.ts.ntiles, std::min<int64_t>(nk / 4, 16));
-  if (want < 2) return false;
+  w.parts = k_pieces(w.ts.ntiles, nk, 4);
+  if (w.parts < 2) return false;
   w.nk_total = nk;
-  w.nk_part = cdiv(nk, want);
-  w.parts = int(cdiv(nk, w.nk_part));
+  w.nk_part = cdiv(nk, int64_t(w.parts));
   void *P = nullptr;
   if (ws_get(WS_PARTS, size_t(w.parts) * size_t(nA) * size_t(nB) * 4, &P) != GT_OK) {
     clear_error();  // no room for the pieces: in one
@@ -1663,7 +1580,7 @@ bool pearson_split(const void *zA, int64_t nA, const void *zB, int64_t nB, int64
     GT_TRY(make_plane_map(&w.mb, zB, nB, kpad, 2, kBN, BK, true));
     GT_TRY((launch_work<tc::KIND_F16X3, BK, true>(w, w.ts.ntiles * w.parts, tc_chunk_kblocks(BK),
                                                   "pearson_gram", s)));
-    pearson_parts_kernel<<<dim3(unsigned(cdiv(nB, 32)), unsigned(cdiv(nA, 32))), 256, 0, s>>>(
+    pearson_parts_kernel<1><<<dim3(unsigned(cdiv(nB, 32)), unsigned(cdiv(nA, 32))), 256, 0, s>>>(
         fin, static_cast<const float *>(P), w.parts);
     count_launch();
     GT_CUDA(cudaGetLastError());
