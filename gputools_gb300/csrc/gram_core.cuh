@@ -220,8 +220,8 @@ inline PairSpace make_pair_space(int64_t nr, int64_t nc, int symmetric, int64_t 
 
 // Band width for operand planes of `panel_bytes` per 256-row B panel: as
 // many B panels as fit in about 48 MB of L2, at most 16 (make_tiles rounds
-// it down to a power of two).  Measured at 20000 x 4096: the error-free Gram
-// (6 MB panels) with groups of 1 / 2 / 4 / 8 / 16 panels 7.13 / 6.91 / 6.76 /
+// it down to a power of two).  Measured at 20000 x 4096 on single CTAs: the error-free
+// Gram (6 MB panels) with groups of 1 / 2 / 4 / 8 / 16 panels 7.13 / 6.91 / 6.76 /
 // 6.59 / 6.74 ms, the f16x3 Gram (4 MB panels) 3.45 ms with 8, 3.52 with 16.
 inline int64_t band_group(int64_t panel_bytes) {
   const char *e = std::getenv("GT_TC_GROUP");
