@@ -219,9 +219,9 @@ gram_exact_kernel(const __grid_constant__ Work work, const tc::WaitCfg wc) {
         }
       }
     }
-    // drain: no bulk copy may still be writing shared memory at exit
-    // (a pair that gives up lets time pass below instead)
-    if (!PAIR && *abort_flag && lead) {
+    // drain: no bulk copy may still be writing shared memory at exit, should another
+    // warp give up later (a pair that gives up lets time pass below instead)
+    if (!PAIR && lead) {
       for (int s = 0; s < kXStages; s++) {
         const int fills = it / kXStages + (s < it % kXStages ? 1 : 0);
         if (fills > 0) tc::mbar_wait_bounded(&full[s], uint32_t((fills - 1) & 1), kDrainLimitNs);

@@ -797,9 +797,9 @@ gram_tc_kernel(const __grid_constant__ Work work, int64_t ckb, const tc::WaitCfg
         __syncwarp();
       }
     }
-    // drain: no bulk copy may still be writing shared memory at exit
-    // (a pair that gives up lets time pass below instead)
-    if (!PAIR && *abort_flag && lead) {
+    // drain: no bulk copy may still be writing shared memory at exit, should another
+    // warp give up later (a pair that gives up lets time pass below instead)
+    if (!PAIR && lead) {
       for (int s = 0; s < C::STAGES; s++) {
         const int fills = it / C::STAGES + (s < it % C::STAGES ? 1 : 0);
         if (fills > 0) tc::mbar_wait_bounded(&full[s], uint32_t((fills - 1) & 1), kDrainLimitNs);

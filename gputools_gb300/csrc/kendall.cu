@@ -302,12 +302,11 @@ kendall_gram_kernel(const __grid_constant__ CUtensorMap ma, const __grid_constan
         tc::tma_load_3d(st, &ma, &full[s], k, int32_t(row0), 0);
         tc::tma_load_3d(st + kSgATile, &mb, &full[s], k, int32_t(col0), 0);
       }
-      // no bulk copy may still be writing shared memory at exit
-      if (*abort_flag) {
-        for (int s = 0; s < kSgStages; s++) {
-          const int fills = it / kSgStages + (s < it % kSgStages ? 1 : 0);
-          if (fills > 0) tc::mbar_wait_bounded(&full[s], uint32_t((fills - 1) & 1), kDrainLimitNs);
-        }
+      // no bulk copy may still be writing shared memory at exit, should another warp
+      // give up later
+      for (int s = 0; s < kSgStages; s++) {
+        const int fills = it / kSgStages + (s < it % kSgStages ? 1 : 0);
+        if (fills > 0) tc::mbar_wait_bounded(&full[s], uint32_t((fills - 1) & 1), kDrainLimitNs);
       }
     }
     __syncwarp();

@@ -236,9 +236,9 @@ pairwise_tc_kernel(const __grid_constant__ PairwiseArgs a, const tc::WaitCfg wc)
         __syncwarp();
       }
     }
-    // drain: no bulk copy may still be writing shared memory at exit (with BOTH
-    // time passes below instead)
-    if (!BOTH && *abort_flag && lead) {
+    // drain: no bulk copy may still be writing shared memory at exit, should another
+    // warp give up later (with BOTH time passes below instead)
+    if (!BOTH && lead) {
       for (int s = 0; s < kPStages; s++) {
         const int fills = it / kPStages + (s < it % kPStages ? 1 : 0);
         if (fills > 0) tc::mbar_wait_bounded(&full[s], uint32_t((fills - 1) & 1), kPDrainNs);
