@@ -333,9 +333,10 @@ kendall_gram_kernel(const __grid_constant__ CUtensorMap ma, const __grid_constan
     }
     if (!ok) *abort_flag = 1;
     // every MMA issued above has finished before the sums are read and TMEM is released
+    // (waited for here too: an epilogue warp may have given up while this one had not)
     if (lead) {
       tc::umma_commit(done);
-      if (!ok) tc::mbar_wait_bounded(done, 0u, kDrainLimitNs);
+      tc::mbar_wait_bounded(done, 0u, kDrainLimitNs);
     }
     __syncwarp();
   } else {
