@@ -227,6 +227,13 @@ gram_exact_kernel(const __grid_constant__ Work work, const tc::WaitCfg wc) {
         if (fills > 0) tc::mbar_wait_bounded(&full[s], uint32_t((fills - 1) & 1), kDrainLimitNs);
       }
     }
+    // ... nor may a pair's multiplies still have to arrive on a stage's barrier here
+    if (PAIR && go && lead) {
+      for (int s = 0; s < kXStages; s++) {
+        const int fills = it / kXStages + (s < it % kXStages ? 1 : 0);
+        if (fills > 0) tc::mbar_wait(&empty[s], uint32_t((fills - 1) & 1), abort_flag, wc);
+      }
+    }
     __syncwarp();
   } else if (warp == 1) {
     // -------------------------------------------------- MMA issuer
@@ -288,12 +295,11 @@ gram_exact_kernel(const __grid_constant__ Work work, const tc::WaitCfg wc) {
     }
     if (!ok) *abort_flag = 1;
     // every MMA issued above has finished before TMEM is released
-    if (lead) {
-      if constexpr (PAIR) {
-        if (rank == 0) tc::umma_commit_pair(mma_done);
-      } else {
-        tc::umma_commit(mma_done);
-      }
+    // (the odd CTA of a pair waits for the arrival below: from here its limit would
+    // run while the even CTA still computes)
+    if (lead && rank == 0) {
+      if constexpr (PAIR) tc::umma_commit_pair(mma_done);
+      else tc::umma_commit(mma_done);
       tc::mbar_wait_bounded(mma_done, 0u, kDrainLimitNs);
     }
     __syncwarp();
@@ -377,6 +383,11 @@ gram_exact_kernel(const __grid_constant__ Work work, const tc::WaitCfg wc) {
     tc::cluster_sync();  // the even CTA's MMAs use both CTAs' memory and arrive in both
   }
   if (warp == 1) {
+    if constexpr (PAIR) {
+      // the last arrival has reached this CTA's memory too
+      if (lane == 0) tc::mbar_wait_bounded(mma_done, 0u, kDrainLimitNs);
+      __syncwarp();
+    }
     tc::tc_fence_after();
     tc::tmem_dealloc<PAIR>(tmem_base, 4 * kXB);
   }
