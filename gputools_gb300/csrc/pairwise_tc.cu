@@ -30,17 +30,11 @@
 // and the pair count from them.
 //
 // The operand copies bound the kernel: 50 KB for the 384 tensor-core cycles of a
-// k-block, 130 bytes a cycle where an SM takes in about 45.  Four fifths are the
-// row variables' planes; with BOTH two CTAs of a cluster take neighbouring column
-// tiles of the same rows and each fetches half of those planes for the two, so
-// that L2 gives them out once (1000 observations of 4000 variables 306 -> 290 us,
-// 200 of 4000 126 -> 111).  Tiles that do not fill the SMs run without it (the
-// cluster's start and end: 100 of 300 36.4 -> 38.9).
+// k-block, 130 bytes a cycle where an SM takes in about 45.
 // Kernel layout as in gram_tc.cu: persistent, one CTA per SM; warp 0 issues
 // the TMA loads, warp 1 the MMAs, warps 2..17 are the epilogue (4 per TMEM
 // lane quarter, 8 column variables each).  Every mbarrier wait is bounded.
 #include "common.cuh"
-#include "gram_core.cuh"
 #include "kernels.cuh"
 #include "stats.cuh"
 #include "tc_ptx.cuh"
@@ -71,8 +65,8 @@ constexpr uint64_t kPDrainNs = 200000000ull;
 constexpr float kPScale = 16384.f;                 // 2^14
 
 struct PairwiseArgs {
-  CUtensorMap ma, mb;  // 3-D maps over the five planes; boxes of 128 (BOTH: 64) and 32 rows
-  const int2 *tiles;   // (first row variable, first column variable) per tile (BOTH: two tiles)
+  CUtensorMap ma, mb;  // 3-D maps over the five planes; boxes of 128 and 32 rows
+  const int2 *tiles;   // (first row variable, first column variable) per tile
   int64_t ntiles, nk;  // tiles, k-blocks
   float *corr, *ts, *pairs;
   int64_t ld, nr, nc;
@@ -160,7 +154,6 @@ __device__ __forceinline__ float signif_pw(float r, float pairs) {
   return r * sqrtf((pairs - 2.f) / (1.f - r * r));
 }
 
-template <bool BOTH>
 __global__ void __launch_bounds__(kPThreads, 1)
 pairwise_tc_kernel(const __grid_constant__ PairwiseArgs a, const tc::WaitCfg wc) {
   if (a.run_if && *a.run_if == 0) return;  // a gated launch whose gate is closed
@@ -176,12 +169,10 @@ pairwise_tc_kernel(const __grid_constant__ PairwiseArgs a, const tc::WaitCfg wc)
   volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int rank = BOTH ? int(tc::cluster_rank()) : 0;
-  const int64_t first = BOTH ? blockIdx.x >> 1 : blockIdx.x, step = BOTH ? gridDim.x >> 1 : gridDim.x;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kPStages; s++) {
       tc::mbar_init(&full[s], 1);
-      tc::mbar_init(&empty[s], BOTH ? 2 : 1);  // every CTA has read the stage
+      tc::mbar_init(&empty[s], 1);
     }
     for (int b = 0; b < 2; b++) {
       tc::mbar_init(&accf[b], 1);
@@ -198,7 +189,6 @@ pairwise_tc_kernel(const __grid_constant__ PairwiseArgs a, const tc::WaitCfg wc)
   if (warp == 1) tc::tmem_alloc(tmem_slot, 512);
   tc::tc_fence_before();
   __syncthreads();
-  if constexpr (BOTH) tc::cluster_sync();  // both CTAs' barriers are there
   tc::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const int64_t nch = (a.nk + kPChunkKb - 1) / kPChunkKb;
@@ -209,9 +199,8 @@ pairwise_tc_kernel(const __grid_constant__ PairwiseArgs a, const tc::WaitCfg wc)
     int it = 0;
     bool go = true;
     const bool lead = tc::elect_one();
-    for (int64_t t = first; t < a.ntiles && go && !*abort_flag; t += step) {
+    for (int64_t t = blockIdx.x; t < a.ntiles && go && !*abort_flag; t += gridDim.x) {
       const int2 tl = a.tiles[t];
-      const int32_t r0 = tl.x + (kPM / 2) * rank, c0 = tl.y + kPN * rank;
       for (int kb = 0; kb < nk; kb++, it++) {
         const int s = it % kPStages;
         go = __all_sync(0xffffffffu, tc::mbar_wait(&empty[s], (uint32_t(it / kPStages) & 1u) ^ 1u,
@@ -224,21 +213,18 @@ pairwise_tc_kernel(const __grid_constant__ PairwiseArgs a, const tc::WaitCfg wc)
         if (lead) {
           tc::mbar_arrive_expect_tx(&full[s], kPStage);
 #pragma unroll
-          for (int p = 0; p < kPlanes; p++) {
-            uint8_t *dst = st + p * kPA + rank * (kPA / 2);
-            if constexpr (BOTH) tc::tma_load_3d_both(dst, &a.ma, &full[s], kb * kPBK, r0, p);
-            else tc::tma_load_3d(dst, &a.ma, &full[s], kb * kPBK, r0, p);
-          }
+          for (int p = 0; p < kPlanes; p++)
+            tc::tma_load_3d(st + p * kPA, &a.ma, &full[s], kb * kPBK, tl.x, p);
 #pragma unroll
           for (int p = 0; p < kPlanes; p++)
-            tc::tma_load_3d(st + kPlanes * kPA + p * kPB, &a.mb, &full[s], kb * kPBK, c0, p);
+            tc::tma_load_3d(st + kPlanes * kPA + p * kPB, &a.mb, &full[s], kb * kPBK, tl.y, p);
         }
         __syncwarp();
       }
     }
     // drain: no bulk copy may still be writing shared memory at exit, should another
-    // warp give up later (with BOTH time passes below instead)
-    if (!BOTH && lead) {
+    // warp give up later
+    if (lead) {
       for (int s = 0; s < kPStages; s++) {
         const int fills = it / kPStages + (s < it % kPStages ? 1 : 0);
         if (fills > 0) tc::mbar_wait_bounded(&full[s], uint32_t((fills - 1) & 1), kPDrainNs);
@@ -257,7 +243,7 @@ pairwise_tc_kernel(const __grid_constant__ PairwiseArgs a, const tc::WaitCfg wc)
     int it = 0, cc = 0;
     bool ok = true;
     const bool lead = tc::elect_one();
-    for (int64_t t = first; t < a.ntiles && ok; t += step) {
+    for (int64_t t = blockIdx.x; t < a.ntiles && ok; t += gridDim.x) {
       for (int kb0 = 0; kb0 < nk && ok; kb0 += int(kPChunkKb), cc++) {
         // two accumulator sets: wait until the epilogue has read the set's
         // previous chunk
@@ -294,8 +280,7 @@ pairwise_tc_kernel(const __grid_constant__ PairwiseArgs a, const tc::WaitCfg wc)
               tc::umma_bf16(d + kR4, aqh, b0, id32, acc);
               tc::umma_bf16(d + kR4, aql, b0, id32, 1u);
             }
-            if constexpr (BOTH) tc::umma_commit_both(&empty[s]);
-            else tc::umma_commit(&empty[s]);
+            tc::umma_commit(&empty[s]);
           }
           __syncwarp();
         }
@@ -316,7 +301,7 @@ pairwise_tc_kernel(const __grid_constant__ PairwiseArgs a, const tc::WaitCfg wc)
     const uint32_t lanes = uint32_t(q * 32) << 16;
     int64_t cc = 0;
     bool ok = true;
-    for (int64_t t = first; t < a.ntiles && ok; t += step) {
+    for (int64_t t = blockIdx.x; t < a.ntiles && ok; t += gridDim.x) {
       const int2 tl = a.tiles[t];
       float sN[8], sA[8], sB[8], sAA[8], sBB[8], sAB[8];
 #pragma unroll
@@ -360,7 +345,7 @@ pairwise_tc_kernel(const __grid_constant__ PairwiseArgs a, const tc::WaitCfg wc)
         if (lane == 0) tc::mbar_arrive(&acce[buf]);
       }
       if (!ok) break;
-      const int64_t r = int64_t(tl.x) + q * 32 + lane, c0 = int64_t(tl.y) + rank * kPN + part * 8;
+      const int64_t r = int64_t(tl.x) + q * 32 + lane, c0 = int64_t(tl.y) + part * 8;
       const float inv = 1.f / kPScale;
 #pragma unroll
       for (int j = 0; j < 8; j++) {  // r into sA, its t-score into sB
@@ -420,14 +405,7 @@ pairwise_tc_kernel(const __grid_constant__ PairwiseArgs a, const tc::WaitCfg wc)
     if (!ok) *abort_flag = 1;
   }
   __syncthreads();
-  if (*abort_flag && threadIdx.x == 0) {
-    atomicOr(wc.err, 1);
-    if (BOTH) tc::pass_time(tc::kCopyTimeNs);  // copies in flight, for both CTAs, end
-  }
-  if constexpr (BOTH) {
-    __syncthreads();
-    tc::cluster_sync();  // the other CTA's copies and commits reach this one's memory
-  }
+  if (*abort_flag && threadIdx.x == 0) atomicOr(wc.err, 1);
   if (warp == 1) {
     tc::tc_fence_after();
     tc::tmem_dealloc(tmem_base, 512);
@@ -442,26 +420,19 @@ pairwise_tc_kernel(const __grid_constant__ PairwiseArgs a, const tc::WaitCfg wc)
 int pearson_pairwise_tc(const float *dA, int64_t nA, const float *dB, int64_t nB, int64_t n,
                         const PearsonOut &out, const int *run_if, cudaStream_t s) {
   if (nA == 0 || nB == 0 || n == 0) return GT_OK;
-  if (nA > 2147483647LL - kPM || nB > 2147483647LL - 2 * kPN)
+  if (nA > 2147483647LL - kPM || nB > 2147483647LL - kPN)
     return fail(GT_EINVAL, "too many variables");
   const bool sym = out.symmetric != 0;
   const int64_t kpad = cdiv(n, 64) * 64;
   const size_t bytesA = size_t(kPlanes) * size_t(nA) * size_t(kpad) * 2;
   const size_t bytesB = sym ? 0 : size_t(kPlanes) * size_t(nB) * size_t(kpad) * 2;
-  // tiles of 128 row variables x 32 column variables, or two of them side by side
-  // where every cluster gets some (see the top); for cor(x) those that reach the
+  // tiles of 128 row variables x 32 column variables; for cor(x) those that reach the
   // upper triangle
   const int64_t tr = cdiv(nA, kPM);
   std::vector<int2> tiles;
-  auto make = [&](int64_t cols) {
-    tiles.clear();
-    for (int64_t ti = 0; ti < tr; ti++)
-      for (int64_t c = sym ? ti * kPM : 0; c < nB; c += cols)
-        tiles.push_back(make_int2(int(ti * kPM), int(c)));
-  };
-  make(2 * kPN);
-  const bool both = 2 * int64_t(tiles.size()) >= sm_count();
-  if (!both) make(kPN);
+  for (int64_t ti = 0; ti < tr; ti++)
+    for (int64_t c = sym ? ti * kPM : 0; c < nB; c += kPN)
+      tiles.push_back(make_int2(int(ti * kPM), int(c)));
   if (tiles.empty()) return GT_OK;
   const size_t tbytes = tiles.size() * sizeof(int2);
   void *pw = nullptr;
@@ -481,7 +452,7 @@ int pearson_pairwise_tc(const float *dA, int64_t nA, const float *dB, int64_t nB
     GT_CUDA(cudaGetLastError());
   }
   PairwiseArgs a{};
-  GT_TRY(tc_plane_map(&a.ma, pa, nA, kpad, kPlanes, both ? kPM / 2 : kPM, kPBK, true));
+  GT_TRY(tc_plane_map(&a.ma, pa, nA, kpad, kPlanes, kPM, kPBK, true));
   GT_TRY(tc_plane_map(&a.mb, pb, nB, kpad, kPlanes, kPN, kPBK, true));
   a.tiles = dtiles;
   a.ntiles = int64_t(tiles.size());
@@ -498,12 +469,11 @@ int pearson_pairwise_tc(const float *dA, int64_t nA, const float *dB, int64_t nB
   GT_TRY(device_error_word(&wc.err));
   wc.limit_ns = wait_limit_ns();
   wc.hint_ns = wait_sleep_hint_ns();
-  auto kern = both ? pairwise_tc_kernel<true> : pairwise_tc_kernel<false>;
-  GT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPSmem));
-  ProfScope prof("pearson_pairwise", s);
-  if (both) return launch_pairs(kern, a.ntiles, kPThreads, kPSmem, s, a, wc);
+  GT_CUDA(cudaFuncSetAttribute(pairwise_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               kPSmem));
   const int64_t grid = a.ntiles < sm_count() ? a.ntiles : sm_count();
-  kern<<<unsigned(grid), kPThreads, kPSmem, s>>>(a, wc);
+  ProfScope prof("pearson_pairwise", s);
+  pairwise_tc_kernel<<<unsigned(grid), kPThreads, kPSmem, s>>>(a, wc);
   count_launch();
   GT_CUDA(cudaGetLastError());
   return GT_OK;

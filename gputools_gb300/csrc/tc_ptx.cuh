@@ -201,18 +201,6 @@ __device__ __forceinline__ void tma_load_3d_pair(void *dst, const CUtensorMap *m
       : "memory");
 }
 
-// The same into both CTAs of a cluster of two: at this offset in each, counted on
-// the barrier at this offset in each.
-__device__ __forceinline__ void tma_load_3d_both(void *dst, const CUtensorMap *map, uint64_t *bar,
-                                                 int32_t c0, int32_t c1, int32_t c2) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      ".multicast::cluster [%0], [%1, {%3, %4, %5}], [%2], %6;" ::"r"(smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2),
-      "h"(uint16_t(3))
-      : "memory");
-}
-
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap *map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
@@ -319,15 +307,6 @@ __device__ __forceinline__ void umma_commit(uint64_t *bar) {
   asm volatile(
       "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
           smem_u32(bar))
-      : "memory");
-}
-
-// The same on the barrier at this offset in both CTAs of a cluster of two.
-__device__ __forceinline__ void umma_commit_both(uint64_t *bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64"
-      " [%0], %1;" ::"r"(smem_u32(bar)),
-      "h"(uint16_t(3))
       : "memory");
 }
 
