@@ -56,6 +56,24 @@ __device__ __forceinline__ void warp_for_each(const float *__restrict__ x, int64
   for (int64_t k = 4 * n4 + lane; k < n; k += 32) f(x[k]);
 }
 
+// The same, four values at a time while there are four: f4(float4), then f.
+template <class F4, class F>
+__device__ __forceinline__ void warp_for_each4(const float *__restrict__ x, int64_t n, F4 &&f4,
+                                               F &&f) {
+  const int lane = threadIdx.x & 31;
+  int64_t done;
+  if ((reinterpret_cast<uintptr_t>(x) & 15u) == 0) {
+    const float4 *x4 = reinterpret_cast<const float4 *>(x);
+    for (int64_t k = lane; k < (n >> 2); k += 32) f4(x4[k]);
+    done = n & ~int64_t(3);
+  } else {
+    done = n & ~int64_t(127);
+    for (int64_t k = lane; k < done; k += 128)
+      f4(make_float4(x[k], x[k + 32], x[k + 64], x[k + 96]));
+  }
+  for (int64_t k = done + lane; k < n; k += 32) f(x[k]);
+}
+
 // Sum of x[0..n) as a float pair in every lane, with the count of non-NaN
 // values, of NaN values, and the largest finite magnitude; values are
 // multiplied by the power of two `sc` first.
@@ -175,14 +193,16 @@ static __device__ __noinline__ ColStats colstats_warp_any(const float *__restric
   return colstats_finish(m, mlo, q, qlo, e, flags);
 }
 
-// colstats_warp_any with fewer instructions a value (11 in the two passes, not
+// colstats_warp_any with fewer instructions a value (18 in the two passes, not
 // 33) for the common variable: every value finite and counted, the plain sum
 // too, fewer than 2^24 values.  The first pass is plain, with the extremes (equal:
-// a constant variable, whose mean is its value); the centred pass sums the
-// residuals plainly and the squares compensated (Kahan, with the products' exact
-// residuals), and is repeated with the corrected mean where the correction is
-// not small (its square beyond 2^-14 of the variance: a mean far above the
-// spread), so that the correction's rounding stays below 2^-36 of the norm.
+// a constant variable, whose mean is its value).  The centred pass sums the
+// residuals four at a time and the squares, with the products' exact residuals, one
+// by one into float pairs: the sum of the squares is good to about 2^-47, beside
+// the rounding of each centred value itself (2^-24 of it, as in colstats_warp_any).
+// It is repeated with the corrected mean where the correction is not small (its
+// square beyond 2^-14 of the variance: a mean far above the spread); a mean that
+// three passes have not settled goes to colstats_warp_any.
 __device__ __forceinline__ ColStats colstats_warp(const float *__restrict__ x, int64_t n,
                                                   int use) {
   const unsigned FULL = 0xffffffffu;
@@ -207,33 +227,38 @@ __device__ __forceinline__ ColStats colstats_warp(const float *__restrict__ x, i
   float m = (s * sc) * invN, mlo = 0.f, q = 0.f, qlo = 0.f;
 #pragma unroll 1
   for (int pass = 0; pass < 3; pass++) {
-    float c = 0.f, ss = 0.f, lost = 0.f;  // the squares sum to ss - lost
-    warp_for_each(x, n, [&](float v) {
+    FloatPairSum c, ss;
+    auto centred = [&](float v) {  // its square goes to ss
       const float d = fmaf(v, sc, -m) - mlo;
-      c += d;
       const float p = d * d;
-      lost -= fmaf(d, d, -p);
-      const float y = p - lost, t = ss + y;
-      lost = (t - ss) - y;
-      ss = t;
-    });
-    q = ss;
-    qlo = -lost;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(FULL, c, o);
+      ss.add(p);
+      ss.lo += fmaf(d, d, -p);
+      return d;
+    };
+    warp_for_each4(
+        x, n,
+        [&](float4 v) {
+          c.add((centred(v.x) + centred(v.y)) + (centred(v.z) + centred(v.w)));
+        },
+        [&](float v) { c.add(centred(v)); });
+    q = ss.hi;
+    qlo = ss.lo;
+    warp_pair_sum(c.hi, c.lo);
     warp_pair_sum(q, qlo);
-    const float cm = c * invN;  // the mean's correction
+    const float C = c.hi + c.lo, cm = C * invN;  // cm: the mean's correction
     mlo += cm;
     const float mean = m + mlo;
     mlo -= mean - m;
     m = mean;
-    const float cc = c * cm;
+    const float cc = C * cm;
     qlo -= cc;
-    if (cc <= 0x1p-14f * q) break;  // (the last pass's sums follow its mean)
+    if (cc <= 0x1p-14f * q) {  // (the sums follow the mean of this pass)
+      const float sum = q + qlo;
+      qlo -= sum - q;
+      return colstats_finish(m, mlo, sum, qlo, e, sum > 0.f ? 0 : 2);
+    }
   }
-  const float sum = q + qlo;
-  qlo -= sum - q;
-  return colstats_finish(m, mlo, sum, qlo, e, sum > 0.f ? 0 : 2);
+  return colstats_warp_any(x, n, use);
 }
 
 // z = (x - mean) * inv_norm in float arithmetic with the mean as a float
