@@ -379,7 +379,7 @@ cor_backward_finish_kernel(const float *__restrict__ X, int64_t p, int64_t n,
     return;
   }
   const Centerer cen(s);
-  const float inv = s.ihi;
+  const float inv = cen.inv;
   float hi = 0.f, lo = 0.f;
   auto acc = [&](float xv, float wv) {
     const float z = cen(xv);

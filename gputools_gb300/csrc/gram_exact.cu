@@ -413,14 +413,16 @@ __device__ __forceinline__ void exact_digits(float vh, float vl, uint16_t (&p)[3
 // (x - mean) * inv_norm * 2^11 as a float pair (about 2^-46 relative), from
 // the statistics, themselves float pairs.
 struct PairCenterer {
-  float mhi, mlo, ihi, ilo;
+  float mhi, mlo, ihi, ilo, sc;
   __device__ __forceinline__ explicit PairCenterer(const ColStats &s) {
-    mhi = s.mhi;
-    mlo = s.mlo;
+    sc = __uint_as_float(uint32_t(127 - s.e) << 23);
+    mhi = s.mhi * sc;
+    mlo = s.mlo * sc;
     ihi = s.ihi * 2048.f;
     ilo = s.ilo * 2048.f;
   }
   __device__ __forceinline__ void operator()(float x, float &vh, float &vl) const {
+    x *= sc;  // a power of two
     // x - mhi exactly (TwoSum), then - mlo into the low part
     const float s = x - mhi;
     const float bp = s - x;

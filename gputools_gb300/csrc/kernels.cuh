@@ -36,9 +36,10 @@ int tc_map_3d(CUtensorMap *map, CUtensorMapDataType type, const void *base,
 // Per-variable statistics of the Pearson prologue.
 struct ColStats {
   float mhi, mlo;  // mean, as a float pair (about 2^-46 relative)
-  float ihi, ilo;  // 1 / sqrt(sum (x - mean)^2) likewise, or 0 for a constant variable
+  float ihi, ilo;  // 2^e / sqrt(sum (x - mean)^2) likewise, or 0 for a constant variable
   int flags;       // bit 0: contains NaN; bit 1: zero variance
-  int unused;
+  int e;           // binade of the largest magnitude, -126 .. 126 (1 / norm itself may
+                   // be subnormal, where a float pair holds few bits)
 };
 
 int launch_colstats(const float *dX, int64_t nvar, int64_t n, int use, ColStats *st,

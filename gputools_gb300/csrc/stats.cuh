@@ -111,12 +111,12 @@ __device__ __forceinline__ WarpSums warp_sums(const float *__restrict__ x, int64
 // times 2^-e).
 __device__ __forceinline__ ColStats colstats_finish(float m, float mlo, float q, float qlo, int e,
                                                     int flags) {
-  const float sc = __uint_as_float(uint32_t(127 - e) << 23);
   const float up = __uint_as_float(uint32_t(127 + e) << 23);
   ColStats st;
   st.mhi = m * up;
   st.mlo = mlo * up;
   st.flags = flags;
+  st.e = e;
   if (flags & 2) {
     st.ihi = st.ilo = 0.f;
   } else {
@@ -124,9 +124,8 @@ __device__ __forceinline__ ColStats colstats_finish(float m, float mlo, float q,
     const float y = rsqrtf(q), y2 = y * y, y2l = fmaf(y, y, -y2);
     const float r = fmaf(-qlo, y2, fmaf(-q, y2l, fmaf(-q, y2, 1.f)));
     const float d = y * r * fmaf(0.375f, r, 0.5f);
-    const float inv = y + d;
-    st.ihi = inv * sc;
-    st.ilo = (d - (inv - y)) * sc;
+    st.ihi = y + d;
+    st.ilo = d - (st.ihi - y);
   }
   return st;
 }
@@ -265,8 +264,9 @@ __device__ __forceinline__ ColStats colstats_warp(const float *__restrict__ x, i
 // pair: the float rounding of the exact value to within a couple of ulp.
 struct Centerer {
   float mhi, mlo, inv;
-  __device__ __forceinline__ explicit Centerer(const ColStats &s)
-      : mhi(s.mhi), mlo(s.mlo), inv(s.ihi) {}
+  __device__ __forceinline__ explicit Centerer(const ColStats &s) : mhi(s.mhi), mlo(s.mlo) {
+    inv = s.ihi * __uint_as_float(uint32_t(127 - s.e) << 23);
+  }
   __device__ __forceinline__ float operator()(float x) const { return ((x - mhi) - mlo) * inv; }
 };
 

@@ -63,3 +63,25 @@ def test_mean_far_above_the_spread_of_many_observations(gpu):
     want = (W - C * (C * W).sum(1, keepdim=True)) / s
     err = (out.double() - want).abs().amax(1) / want.abs().amax(1)
     assert float(err.max()) <= 4e-6
+
+
+@pytest.mark.parametrize("log2scale", [118, 123, -115, -120])
+def test_norms_near_the_ends_of_the_float_range(gpu, rng, log2scale):
+    """1 / norm subnormal, or its low half: the error-free Gram's tolerance all the same."""
+    import torch
+    import gputools_gb300 as g
+    p, n = 24, 1024
+    X = (rng.standard_normal((1, n)) + rng.standard_normal((p, n))).astype(np.float32)
+    Z = X.astype(np.float64)
+    Z -= Z.mean(1, keepdims=True)
+    Z /= np.linalg.norm(Z, axis=1, keepdims=True)
+    want = Z @ Z.T
+    np.fill_diagonal(want, 1.0)
+    dX = torch.from_numpy(X * np.float32(2.0 ** log2scale)).cuda()
+    old = g.get_gram_path()
+    g.set_gram_path("f16x6")
+    try:
+        got = g.pmcc_device(dX, outputs=("corr",))["corr"].cpu().numpy()
+    finally:
+        g.set_gram_path(old)
+    assert np.max(np.abs(got - want)) <= 1.5e-7
