@@ -719,6 +719,10 @@ struct PtPartials {
   double *loss;  // one per segment
 };
 
+// W of a pair with a NaN coordinate: the pair adds nothing to the gradient (a NaN
+// that no operation makes).
+constexpr int kPtNone = 0x7fc0abcd;
+
 __host__ __device__ inline int64_t pt_first(int64_t I, int64_t nb) { return I * nb - I * (I - 1) / 2; }
 
 template <int DMAX, int MODE>
@@ -807,6 +811,7 @@ dist_pairs_kernel(const float *__restrict__ X, int64_t n, int64_t dim,
     if (t + 1 < t1) load(xj + (b ^ 1) * L::X, (row_ends ? I + 1 : J + 1) * kPtT);
     const float *xb = xj + b * L::X;
     // ------------------------------------------------ phase 1, two columns at a time
+    bool none = false;
     auto phase1 = [&](auto inner) {
       constexpr bool INNER = decltype(inner)::value;  // every pair i < j < n
 #pragma unroll 1
@@ -876,6 +881,10 @@ dist_pairs_kernel(const float *__restrict__ X, int64_t n, int64_t dim,
               }
               // coincident points add to the stress but not to the gradient
               if (d2 > 0.f) w = MODE == 0 ? cf[a][c] * inv_d : 2.f * (d - cf[a][c]) * inv_d;
+              if (d2 != d2) {
+                w = __int_as_float(kPtNone);
+                none = true;
+              }
             }
             ws[il * L::LW + jl] = w;
             wt[jl * L::LT + il] = w;
@@ -884,7 +893,7 @@ dist_pairs_kernel(const float *__restrict__ X, int64_t n, int64_t dim,
     };
     if (I < J && j0 + kPtT <= n) phase1(std::true_type{});
     else phase1(std::false_type{});
-    __syncthreads();
+    const bool skips = __syncthreads_or(none);
     // ------------------------------------------------ phase 2
 #pragma unroll
     for (int r = 0; r < 4; r++) {
@@ -917,10 +926,29 @@ dist_pairs_kernel(const float *__restrict__ X, int64_t n, int64_t dim,
         }
       }
     };
+    if (!skips) {
 #pragma unroll 1
-    for (int q = 0; q < 4; q++) {  // a quarter of the sums of W in each warp
-      if (q == w4) rows16(16 * q, std::true_type{});
-      else rows16(16 * q, std::false_type{});
+      for (int q = 0; q < 4; q++) {  // a quarter of the sums of W in each warp
+        if (q == w4) rows16(16 * q, std::true_type{});
+        else rows16(16 * q, std::false_type{});
+      }
+    } else {  // a NaN coordinate in the tile: only the pairs that count (0 * NaN would not be 0)
+#pragma unroll 1
+      for (int m = 0; m < kPtT; m++) {
+#pragma unroll 1
+        for (int r = 0; r < 4; r++) {
+          const float w = pw[m * lw + r];
+          const int64_t i = i0 + (side ? m : 4 * rg + r), j = j0 + (side ? 4 * rg + r : m);
+          if (i >= j || j >= n || __float_as_int(w) == kPtNone) continue;
+#pragma unroll
+          for (int q = 0; q < 4; q++) {
+            if (q != r) continue;
+#pragma unroll
+            for (int k = 0; k < DPT; k++) acc[q][k] = fmaf(w, px[m * L::LD + k], acc[q][k]);
+            if (m >> 4 == w4) wsum[q] += w;
+          }
+        }
+      }
     }
     const bool flush_row = row_ends || t + 1 == t1;  // uniform
     if (side == 1) {
