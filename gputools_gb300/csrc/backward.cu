@@ -298,7 +298,7 @@ template <class T>
 __global__ void zt_operand_kernel(const float *__restrict__ X, int64_t p, int64_t n, int64_t kp,
                                   const ColStats *__restrict__ st, int ns, T *__restrict__ Zt) {
   __shared__ float tile[32][33];
-  __shared__ float cen[32][4];  // the block's 32 variables: mean pair, inverse norm, flag
+  __shared__ float cen[32][5];  // the block's 32 variables: mean pair, inverse norm, scale, flag
   const int64_t k0 = int64_t(blockIdx.x) * 32, i0 = int64_t(blockIdx.y) * 32;
   const int tx = threadIdx.x, ty0 = threadIdx.y;
   if (ty0 == 0) {
@@ -309,15 +309,16 @@ __global__ void zt_operand_kernel(const float *__restrict__ X, int64_t p, int64_
       cen[tx][0] = c.mhi;
       cen[tx][1] = c.mlo;
       cen[tx][2] = c.inv;
-      cen[tx][3] = s.flags ? 1.f : 0.f;
+      cen[tx][3] = c.sc;
+      cen[tx][4] = s.flags ? 1.f : 0.f;
     }
   }
   __syncthreads();
   for (int ty = ty0; ty < 32; ty += 8) {
     const int64_t i = i0 + ty, k = k0 + tx;
     float z = 0.f;
-    if (i < p && k < n && cen[ty][3] == 0.f)
-      z = ((X[i * n + k] - cen[ty][0]) - cen[ty][1]) * cen[ty][2];
+    if (i < p && k < n && cen[ty][4] == 0.f)
+      z = (fmaf(X[i * n + k], cen[ty][3], -cen[ty][0]) - cen[ty][1]) * cen[ty][2];
     tile[ty][tx] = z;  // rows i
   }
   __syncthreads();
@@ -379,7 +380,7 @@ cor_backward_finish_kernel(const float *__restrict__ X, int64_t p, int64_t n,
     return;
   }
   const Centerer cen(s);
-  const float inv = cen.inv;
+  const float inv = cen.inv * cen.sc;
   float hi = 0.f, lo = 0.f;
   auto acc = [&](float xv, float wv) {
     const float z = cen(xv);

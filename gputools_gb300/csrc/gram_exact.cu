@@ -415,9 +415,9 @@ __device__ __forceinline__ void exact_digits(float vh, float vl, uint16_t (&p)[3
 struct PairCenterer {
   float mhi, mlo, ihi, ilo, sc;
   __device__ __forceinline__ explicit PairCenterer(const ColStats &s) {
-    sc = __uint_as_float(uint32_t(127 - s.e) << 23);
-    mhi = s.mhi * sc;
-    mlo = s.mlo * sc;
+    sc = s.scale();
+    mhi = s.mhi;
+    mlo = s.mlo;
     ihi = s.ihi * 2048.f;
     ilo = s.ilo * 2048.f;
   }

@@ -33,13 +33,17 @@ int tc_map_3d(CUtensorMap *map, CUtensorMapDataType type, const void *base,
               const cuuint64_t (&dims)[3], const cuuint64_t (&strides)[2],
               const cuuint32_t (&box)[3], CUtensorMapSwizzle swizzle);
 
-// Per-variable statistics of the Pearson prologue.
+// Per-variable statistics of the Pearson prologue, of the values times 2^-e: the
+// inverse norm of the values themselves may be subnormal, where a float pair holds few
+// bits, or beyond the float range.
 struct ColStats {
   float mhi, mlo;  // mean, as a float pair (about 2^-46 relative)
-  float ihi, ilo;  // 2^e / sqrt(sum (x - mean)^2) likewise, or 0 for a constant variable
+  float ihi, ilo;  // 1 / sqrt(sum (x - mean)^2) likewise, or 0 for a constant variable
   int flags;       // bit 0: contains NaN; bit 1: zero variance
-  int e;           // binade of the largest magnitude, -126 .. 126 (1 / norm itself may
-                   // be subnormal, where a float pair holds few bits)
+  int e;           // binade of the largest magnitude, -126 .. 126
+  __device__ __forceinline__ float scale() const {  // 2^-e
+    return __uint_as_float(uint32_t(127 - e) << 23);
+  }
 };
 
 int launch_colstats(const float *dX, int64_t nvar, int64_t n, int use, ColStats *st,

@@ -111,10 +111,9 @@ __device__ __forceinline__ WarpSums warp_sums(const float *__restrict__ x, int64
 // times 2^-e).
 __device__ __forceinline__ ColStats colstats_finish(float m, float mlo, float q, float qlo, int e,
                                                     int flags) {
-  const float up = __uint_as_float(uint32_t(127 + e) << 23);
   ColStats st;
-  st.mhi = m * up;
-  st.mlo = mlo * up;
+  st.mhi = m;
+  st.mlo = mlo;
   st.flags = flags;
   st.e = e;
   if (flags & 2) {
@@ -263,11 +262,12 @@ __device__ __forceinline__ ColStats colstats_warp(const float *__restrict__ x, i
 // z = (x - mean) * inv_norm in float arithmetic with the mean as a float
 // pair: the float rounding of the exact value to within a couple of ulp.
 struct Centerer {
-  float mhi, mlo, inv;
-  __device__ __forceinline__ explicit Centerer(const ColStats &s) : mhi(s.mhi), mlo(s.mlo) {
-    inv = s.ihi * __uint_as_float(uint32_t(127 - s.e) << 23);
+  float mhi, mlo, inv, sc;  // of the values times sc, a power of two
+  __device__ __forceinline__ explicit Centerer(const ColStats &s)
+      : mhi(s.mhi), mlo(s.mlo), inv(s.ihi), sc(s.scale()) {}
+  __device__ __forceinline__ float operator()(float x) const {
+    return (fmaf(x, sc, -mhi) - mlo) * inv;
   }
-  __device__ __forceinline__ float operator()(float x) const { return ((x - mhi) - mlo) * inv; }
 };
 
 }  // namespace gt

@@ -85,3 +85,24 @@ def test_norms_near_the_ends_of_the_float_range(gpu, rng, log2scale):
     finally:
         g.set_gram_path(old)
     assert np.max(np.abs(got - want)) <= 1.5e-7
+
+
+@pytest.mark.parametrize("path", ["f16x3", "fp32", "f16x6"])
+@pytest.mark.parametrize("p,n", [(24, 64), (300, 40)])
+def test_subnormal_values(gpu, rng, path, p, n):
+    """Whole multiples of the smallest float: exact inputs of which 1 / norm overflows."""
+    import torch
+    import gputools_gb300 as g
+    K = (rng.integers(-500, 500, (1, n)) + rng.integers(-500, 500, (p, n))).astype(np.float64)
+    X = (K * 2.0 ** -149).astype(np.float32)
+    Z = K - K.mean(1, keepdims=True)
+    Z /= np.linalg.norm(Z, axis=1, keepdims=True)
+    want = Z @ Z.T
+    np.fill_diagonal(want, 1.0)
+    old = g.get_gram_path()
+    g.set_gram_path(path)
+    try:
+        got = g.pmcc_device(torch.from_numpy(X).cuda(), outputs=("corr",))["corr"].cpu().numpy()
+    finally:
+        g.set_gram_path(old)
+    assert np.max(np.abs(got - want)) <= (1.5e-7 if path == "f16x6" else 3e-6)
