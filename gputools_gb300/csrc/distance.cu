@@ -196,7 +196,8 @@ struct OpValue {
 // so it is read as +Inf.  Coordinates where both points are zero are counted
 // at the end from the points' packed nonzero bits, 32 to a popcount.  From the
 // first slab with a huge, tiny or non-finite value on (voted by the barrier
-// that ends the slab before it) a tile takes the divisions.
+// that ends the slab before it) a tile takes the divisions, on the values
+// themselves.
 // Bound by the FMA pipe: 16000 x 64, a tenth zeros, dist layout: 1.53 ms (9.54
 // before, 4.4 of them the two FP64 divisions of each rescaled entry).
 constexpr float kCanZero = 0x1p-60f, kCanLo = 0x1p-30f, kCanHi = 0x1p60f;
@@ -213,9 +214,10 @@ __device__ __forceinline__ float canberra_finish(float sum, int zeros, int64_t K
   return q + __fdividef(fmaf(-q, used, p) + pe, used);
 }
 
-// Replaces a chunk's zeros; whether a value is out of the range.
+// Replaces a chunk's zeros (noted in the next bits of `zeros`); whether a value is out
+// of the range.
 template <int CHUNKS>
-__device__ __forceinline__ bool canberra_prepare(float4 (&r)[CHUNKS]) {
+__device__ __forceinline__ bool canberra_prepare(float4 (&r)[CHUNKS], unsigned &zeros) {
   bool bad = false;
 #pragma unroll
   for (int s = 0; s < CHUNKS; s++) {
@@ -225,6 +227,7 @@ __device__ __forceinline__ bool canberra_prepare(float4 (&r)[CHUNKS]) {
       const bool zero = e[i] == 0.f;
       bad |= !(zero || (fabsf(e[i]) >= kCanLo && fabsf(e[i]) <= kCanHi));
       if (zero) e[i] = kCanZero;
+      zeros = 2 * zeros + zero;
     }
   }
   return bad;
@@ -254,109 +257,116 @@ canberra_kernel(SimtArgs a, const unsigned *__restrict__ bits, int64_t words,
   float4 ra[BM * 4 / kSimtThreads], rb[BN * 4 / kSimtThreads];
   simt_load<BM, OpEuclid>(ra, a.R, a.ldr, a.nr, row0, 0, a.K, a.vec_ok);
   simt_load<BN, OpEuclid>(rb, a.C, a.ldc, a.nc, col0, 0, a.K, a.vec_ok);
-  bool bad = canberra_prepare(ra);
-  bad |= canberra_prepare(rb);
-  simt_store<BM, false>(sA[0], ra);
-  simt_store<BN, true>(sB[0], rb);
-  bool divide = __syncthreads_or(bad);  // uniform; stays set
-  auto settle = [&] {  // the end of the slabs without divisions
+  // The slab in ra, rb to buffer b, its zeros replaced; true if a value is out of the
+  // range (uniform): then the slab is stored as it is.
+  auto store = [&](int b) {
+    unsigned zeros = 0;
+    bool bad = canberra_prepare(ra, zeros);
+    bad |= canberra_prepare(rb, zeros);
+    simt_store<BM, false>(sA[b], ra);
+    simt_store<BN, true>(sB[b], rb);
+    if (!__syncthreads_or(bad)) return false;
+    static_assert(BM * 4 == kSimtThreads && BN * 4 == kSimtThreads, "a chunk a thread");
 #pragma unroll
-    for (int i = 0; i < TM; i++)
-#pragma unroll
-      for (int j = 0; j < TN / 2; j++) {
-        if (acc[i][j].x != acc[i][j].x) acc[i][j].x = __int_as_float(0x7f800000);
-        if (acc[i][j].y != acc[i][j].y) acc[i][j].y = __int_as_float(0x7f800000);
-      }
+    for (int i = 0; i < 4; i++) {
+      if ((zeros >> (7 - i)) & 1u) (&ra[0].x)[i] = 0.f;
+      if ((zeros >> (3 - i)) & 1u) (&rb[0].x)[i] = 0.f;
+    }
+    simt_store<BM, false>(sA[b], ra);
+    simt_store<BN, true>(sB[b], rb);
+    __syncthreads();
+    return true;
   };
-
-  const int64_t nk = (a.K + kSimtBK - 1) / kSimtBK;
-  for (int64_t kb = 0; kb < nk; kb++) {
-    const int buf = int(kb & 1);
+  bool divide = store(0);
+  const int nk = int((a.K + kSimtBK - 1) / kSimtBK);
+  int kb = 0;
+  for (; kb < nk && !divide; kb++) {
+    const int buf = kb & 1;
     const bool more = kb + 1 < nk;
     if (more) {
-      simt_load<BM, OpEuclid>(ra, a.R, a.ldr, a.nr, row0, (kb + 1) * kSimtBK, a.K, a.vec_ok);
-      simt_load<BN, OpEuclid>(rb, a.C, a.ldc, a.nc, col0, (kb + 1) * kSimtBK, a.K, a.vec_ok);
+      simt_load<BM, OpEuclid>(ra, a.R, a.ldr, a.nr, row0, int64_t(kb + 1) * kSimtBK, a.K, a.vec_ok);
+      simt_load<BN, OpEuclid>(rb, a.C, a.ldc, a.nc, col0, int64_t(kb + 1) * kSimtBK, a.K, a.vec_ok);
     }
     const float *pa = sA[buf] + 4 * ty, *pb = sB[buf] + 4 * tx;
-    if (!divide) {
-      const float2 minus = make_float2(-1.f, -1.f);
-      const int kend = a.K - kb * kSimtBK < kSimtBK ? int(a.K - kb * kSimtBK) : kSimtBK;
+    const float2 minus = make_float2(-1.f, -1.f);
+    const int left = int(a.K - int64_t(kb) * kSimtBK), kend = left < kSimtBK ? left : kSimtBK;
 #pragma unroll 2
-      for (int kk = 0; kk < kend; kk += 2) {  // an odd last term pairs with padding, 0 / 2^-59
-        float2 y0[TN / 2], y1[TN / 2];
+    for (int kk = 0; kk < kend; kk += 2) {  // an odd last term pairs with padding, 0 / 2^-59
+      float2 y0[TN / 2], y1[TN / 2];
 #pragma unroll
-        for (int g = 0; g < TN / 4; g++) {
-          const float4 u = *reinterpret_cast<const float4 *>(pb + kk * LDB + 64 * g);
-          const float4 v = *reinterpret_cast<const float4 *>(pb + (kk + 1) * LDB + 64 * g);
-          y0[2 * g] = make_float2(u.x, u.y);
-          y0[2 * g + 1] = make_float2(u.z, u.w);
-          y1[2 * g] = make_float2(v.x, v.y);
-          y1[2 * g + 1] = make_float2(v.z, v.w);
-        }
-#pragma unroll
-        for (int g = 0; g < TM / 4; g++) {
-          const float4 u = *reinterpret_cast<const float4 *>(pa + kk * LDA + 64 * g);
-          const float4 v = *reinterpret_cast<const float4 *>(pa + (kk + 1) * LDA + 64 * g);
-#pragma unroll
-          for (int e = 0; e < 4; e++) {
-            const float2 x0 = make_float2((&u.x)[e], (&u.x)[e]);
-            const float2 x1 = make_float2((&v.x)[e], (&v.x)[e]);
-#pragma unroll
-            for (int j = 0; j < TN / 2; j++) {
-              const float2 d0 = __fadd2_rn(x0, y0[j]), d1 = __fadd2_rn(x1, y1[j]);
-              const float2 p0 = __fmul2_rn(__ffma2_rn(y0[j], minus, x0), d1);
-              const float2 p1 = __fmul2_rn(__ffma2_rn(y1[j], minus, x1), d0);
-              const float2 n = make_float2(fabsf(p0.x) + fabsf(p1.x), fabsf(p0.y) + fabsf(p1.y));
-              const float2 d = __fmul2_rn(d0, d1);
-              float2 inv;
-              asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv.x) : "f"(fabsf(d.x)));
-              asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv.y) : "f"(fabsf(d.y)));
-              acc[4 * g + e][j] = __ffma2_rn(n, inv, acc[4 * g + e][j]);
-            }
-          }
-        }
-      }
-    } else {
-      // bit kk: coordinate kk of the slab is nonzero (rows and columns past
-      // the end are never stored)
-      unsigned za[TM], zb[TN];
-#pragma unroll
-      for (int i = 0; i < TM; i++) {
-        const int64_t r = row0 + simt_row(i, ty);
-        za[i] = r < a.nr ? bits[r * words + (kb >> 1)] >> (16 * (kb & 1)) : 0u;
+      for (int g = 0; g < TN / 4; g++) {
+        const float4 u = *reinterpret_cast<const float4 *>(pb + kk * LDB + 64 * g);
+        const float4 v = *reinterpret_cast<const float4 *>(pb + (kk + 1) * LDB + 64 * g);
+        y0[2 * g] = make_float2(u.x, u.y);
+        y0[2 * g + 1] = make_float2(u.z, u.w);
+        y1[2 * g] = make_float2(v.x, v.y);
+        y1[2 * g + 1] = make_float2(v.z, v.w);
       }
 #pragma unroll
-      for (int j = 0; j < TN; j++) {
-        const int64_t c = col0 + tx + 16 * j;
-        zb[j] = c < a.nc ? bits[c * words + (kb >> 1)] >> (16 * (kb & 1)) : 0u;
-      }
-#pragma unroll 1
-      for (int kk = 0; kk < kSimtBK; kk++) {
-        if (kb * kSimtBK + kk >= a.K) break;
+      for (int g = 0; g < TM / 4; g++) {
+        const float4 u = *reinterpret_cast<const float4 *>(pa + kk * LDA + 64 * g);
+        const float4 v = *reinterpret_cast<const float4 *>(pa + (kk + 1) * LDA + 64 * g);
 #pragma unroll
-        for (int i = 0; i < TM; i++) {
-          const bool ui = (za[i] >> kk) & 1u;
-          const float x = ui ? pa[kk * LDA + 64 * (i >> 2) + (i & 3)] : 0.f;
+        for (int e = 0; e < 4; e++) {
+          const float2 x0 = make_float2((&u.x)[e], (&u.x)[e]);
+          const float2 x1 = make_float2((&v.x)[e], (&v.x)[e]);
 #pragma unroll
-          for (int j = 0; j < TN; j++) {
-            const bool uj = (zb[j] >> kk) & 1u;
-            const float y = uj ? pb[kk * LDB + 64 * (j >> 2) + (j & 3)] : 0.f;
-            float &s = j & 1 ? acc[i][j / 2].y : acc[i][j / 2].x;
-            if (ui || uj) s += __fdiv_rn(fabsf(x - y), fabsf(x + y));
+          for (int j = 0; j < TN / 2; j++) {
+            const float2 d0 = __fadd2_rn(x0, y0[j]), d1 = __fadd2_rn(x1, y1[j]);
+            const float2 p0 = __fmul2_rn(__ffma2_rn(y0[j], minus, x0), d1);
+            const float2 p1 = __fmul2_rn(__ffma2_rn(y1[j], minus, x1), d0);
+            const float2 n = make_float2(fabsf(p0.x) + fabsf(p1.x), fabsf(p0.y) + fabsf(p1.y));
+            const float2 d = __fmul2_rn(d0, d1);
+            float2 inv;
+            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv.x) : "f"(fabsf(d.x)));
+            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv.y) : "f"(fabsf(d.y)));
+            acc[4 * g + e][j] = __ffma2_rn(n, inv, acc[4 * g + e][j]);
           }
         }
       }
     }
-    bad = false;
+    if (more) divide = store(buf ^ 1);
+    else __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < TM; i++)  // the slabs without divisions end
+#pragma unroll
+    for (int j = 0; j < TN / 2; j++) {
+      if (acc[i][j].x != acc[i][j].x) acc[i][j].x = __int_as_float(0x7f800000);
+      if (acc[i][j].y != acc[i][j].y) acc[i][j].y = __int_as_float(0x7f800000);
+    }
+  for (; kb < nk; kb++) {
+    const int buf = kb & 1;
+    const bool more = kb + 1 < nk;
     if (more) {
-      bad = canberra_prepare(ra);
-      bad |= canberra_prepare(rb);
+      simt_load<BM, OpEuclid>(ra, a.R, a.ldr, a.nr, row0, int64_t(kb + 1) * kSimtBK, a.K, a.vec_ok);
+      simt_load<BN, OpEuclid>(rb, a.C, a.ldc, a.nc, col0, int64_t(kb + 1) * kSimtBK, a.K, a.vec_ok);
+    }
+    const float *pa = sA[buf] + 4 * ty, *pb = sB[buf] + 4 * tx;
+    const int left = int(a.K - int64_t(kb) * kSimtBK), kend = left < kSimtBK ? left : kSimtBK;
+#pragma unroll 2
+    for (int kk = 0; kk < kend; kk++) {
+      const float4 u = *reinterpret_cast<const float4 *>(pa + kk * LDA);
+      const float4 v = *reinterpret_cast<const float4 *>(pb + kk * LDB);
+#pragma unroll
+      for (int i = 0; i < TM; i++) {
+#pragma unroll
+        for (int j = 0; j < TN; j++) {
+          const float x = (&u.x)[i], y = (&v.x)[j];
+          const float num = fabsf(x - y), den = fabsf(x + y);
+          // equal values add 0, zeros among them (a division of 0 takes its slow path)
+          const bool same = num == 0.f;
+          const float t = __fdiv_rn(same ? 1.f : num, same ? 1.f : den);
+          float &sum = j & 1 ? acc[i][j / 2].y : acc[i][j / 2].x;
+          sum += same ? 0.f : t;
+        }
+      }
+    }
+    if (more) {
       simt_store<BM, false>(sA[buf ^ 1], ra);
       simt_store<BN, true>(sB[buf ^ 1], rb);
     }
-    const bool next = __syncthreads_or(bad) || divide;
-    if ((next || !more) && !divide) settle();
-    divide = next;
+    __syncthreads();
   }
 
   // coordinates where both points are zero: all but those nonzero in either
