@@ -197,10 +197,13 @@ struct OpValue {
 // at the end from the points' packed nonzero bits, 32 to a popcount.  From the
 // first slab with a huge, tiny or non-finite value on (voted by the barrier
 // that ends the slab before it) a tile takes the divisions, on the values
-// themselves.
+// themselves.  Fewer than 8 coordinates (FEW), whose additions do not make up for the
+// roundings of a shared denominator, take a reciprocal a term and correct the quotient
+// by its residual (about half an ulp, as the division).
 // Bound by the FMA pipe: 16000 x 64, a tenth zeros, dist layout: 1.53 ms (9.54
 // before, 4.4 of them the two FP64 divisions of each rescaled entry).
 constexpr float kCanZero = 0x1p-60f, kCanLo = 0x1p-30f, kCanHi = 0x1p60f;
+constexpr int kCanMinK = 8;
 
 // sum * dim / used with one rounding (the product's and the quotient's
 // residuals are added back) where the product cannot overflow.
@@ -237,6 +240,7 @@ __device__ __forceinline__ bool canberra_prepare(float4 (&r)[CHUNKS], unsigned &
 // 64 x 64 tiles, three blocks an SM: 128 x 128 tiles with two blocks or one
 // measured 1.51 and 1.87 ms where these took 1.49, and 215 / 236 us against 185
 // at 4000 x 100 (full).
+template <bool FEW>
 __global__ void __launch_bounds__(kSimtThreads, 3)
 canberra_kernel(SimtArgs a, const unsigned *__restrict__ bits, int64_t words,
                 OutDist<OpValue> out) {
@@ -288,39 +292,64 @@ canberra_kernel(SimtArgs a, const unsigned *__restrict__ bits, int64_t words,
       simt_load<BN, OpEuclid>(rb, a.C, a.ldc, a.nc, col0, int64_t(kb + 1) * kSimtBK, a.K, a.vec_ok);
     }
     const float *pa = sA[buf] + 4 * ty, *pb = sB[buf] + 4 * tx;
-    const float2 minus = make_float2(-1.f, -1.f);
-    const int left = int(a.K - int64_t(kb) * kSimtBK), kend = left < kSimtBK ? left : kSimtBK;
+    if constexpr (FEW) {
+      const float2 minus = make_float2(-1.f, -1.f);
 #pragma unroll 2
-    for (int kk = 0; kk < kend; kk += 2) {  // an odd last term pairs with padding, 0 / 2^-59
-      float2 y0[TN / 2], y1[TN / 2];
+      for (int kk = 0; kk < int(a.K); kk++) {
+        const float4 u = *reinterpret_cast<const float4 *>(pa + kk * LDA);
+        const float4 v = *reinterpret_cast<const float4 *>(pb + kk * LDB);
+        const float2 y[2] = {make_float2(v.x, v.y), make_float2(v.z, v.w)};
 #pragma unroll
-      for (int g = 0; g < TN / 4; g++) {
-        const float4 u = *reinterpret_cast<const float4 *>(pb + kk * LDB + 64 * g);
-        const float4 v = *reinterpret_cast<const float4 *>(pb + (kk + 1) * LDB + 64 * g);
-        y0[2 * g] = make_float2(u.x, u.y);
-        y0[2 * g + 1] = make_float2(u.z, u.w);
-        y1[2 * g] = make_float2(v.x, v.y);
-        y1[2 * g + 1] = make_float2(v.z, v.w);
-      }
-#pragma unroll
-      for (int g = 0; g < TM / 4; g++) {
-        const float4 u = *reinterpret_cast<const float4 *>(pa + kk * LDA + 64 * g);
-        const float4 v = *reinterpret_cast<const float4 *>(pa + (kk + 1) * LDA + 64 * g);
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-          const float2 x0 = make_float2((&u.x)[e], (&u.x)[e]);
-          const float2 x1 = make_float2((&v.x)[e], (&v.x)[e]);
+        for (int i = 0; i < TM; i++) {
+          const float2 x = make_float2((&u.x)[i], (&u.x)[i]);
 #pragma unroll
           for (int j = 0; j < TN / 2; j++) {
-            const float2 d0 = __fadd2_rn(x0, y0[j]), d1 = __fadd2_rn(x1, y1[j]);
-            const float2 p0 = __fmul2_rn(__ffma2_rn(y0[j], minus, x0), d1);
-            const float2 p1 = __fmul2_rn(__ffma2_rn(y1[j], minus, x1), d0);
-            const float2 n = make_float2(fabsf(p0.x) + fabsf(p1.x), fabsf(p0.y) + fabsf(p1.y));
-            const float2 d = __fmul2_rn(d0, d1);
+            float2 d = __fadd2_rn(x, y[j]), n = __ffma2_rn(y[j], minus, x);
+            n = make_float2(fabsf(n.x), fabsf(n.y));
+            d = make_float2(-fabsf(d.x), -fabsf(d.y));
             float2 inv;
-            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv.x) : "f"(fabsf(d.x)));
-            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv.y) : "f"(fabsf(d.y)));
-            acc[4 * g + e][j] = __ffma2_rn(n, inv, acc[4 * g + e][j]);
+            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv.x) : "f"(-d.x));
+            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv.y) : "f"(-d.y));
+            const float2 q = __fmul2_rn(n, inv);
+            acc[i][j] = __fadd2_rn(acc[i][j], __ffma2_rn(__ffma2_rn(q, d, n), inv, q));
+          }
+        }
+      }
+    } else {
+      const float2 minus = make_float2(-1.f, -1.f);
+      const int left = int(a.K - int64_t(kb) * kSimtBK), kend = left < kSimtBK ? left : kSimtBK;
+#pragma unroll 2
+      for (int kk = 0; kk < kend; kk += 2) {  // an odd last term pairs with padding, 0 / 2^-59
+        float2 y0[TN / 2], y1[TN / 2];
+#pragma unroll
+        for (int g = 0; g < TN / 4; g++) {
+          const float4 u = *reinterpret_cast<const float4 *>(pb + kk * LDB + 64 * g);
+          const float4 v = *reinterpret_cast<const float4 *>(pb + (kk + 1) * LDB + 64 * g);
+          y0[2 * g] = make_float2(u.x, u.y);
+          y0[2 * g + 1] = make_float2(u.z, u.w);
+          y1[2 * g] = make_float2(v.x, v.y);
+          y1[2 * g + 1] = make_float2(v.z, v.w);
+        }
+#pragma unroll
+        for (int g = 0; g < TM / 4; g++) {
+          const float4 u = *reinterpret_cast<const float4 *>(pa + kk * LDA + 64 * g);
+          const float4 v = *reinterpret_cast<const float4 *>(pa + (kk + 1) * LDA + 64 * g);
+#pragma unroll
+          for (int e = 0; e < 4; e++) {
+            const float2 x0 = make_float2((&u.x)[e], (&u.x)[e]);
+            const float2 x1 = make_float2((&v.x)[e], (&v.x)[e]);
+#pragma unroll
+            for (int j = 0; j < TN / 2; j++) {
+              const float2 d0 = __fadd2_rn(x0, y0[j]), d1 = __fadd2_rn(x1, y1[j]);
+              const float2 p0 = __fmul2_rn(__ffma2_rn(y0[j], minus, x0), d1);
+              const float2 p1 = __fmul2_rn(__ffma2_rn(y1[j], minus, x1), d0);
+              const float2 n = make_float2(fabsf(p0.x) + fabsf(p1.x), fabsf(p0.y) + fabsf(p1.y));
+              const float2 d = __fmul2_rn(d0, d1);
+              float2 inv;
+              asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv.x) : "f"(fabsf(d.x)));
+              asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv.y) : "f"(fabsf(d.y)));
+              acc[4 * g + e][j] = __ffma2_rn(n, inv, acc[4 * g + e][j]);
+            }
           }
         }
       }
@@ -419,7 +448,10 @@ cudaError_t run_canberra(const float *pts, const unsigned *bits, int64_t n, int6
   const SimtArgs a = dist_args(pts, n, dim);
   const OutDist<OpValue> o{OpValue{}, out, n, dim, layout};
   const unsigned g = unsigned(cdiv(n, 64));
-  canberra_kernel<<<dim3(g, g), kSimtThreads, 0, st>>>(a, bits, cdiv(dim, 32), o);
+  if (dim < kCanMinK)
+    canberra_kernel<true><<<dim3(g, g), kSimtThreads, 0, st>>>(a, bits, cdiv(dim, 32), o);
+  else
+    canberra_kernel<false><<<dim3(g, g), kSimtThreads, 0, st>>>(a, bits, cdiv(dim, 32), o);
   count_launch();
   return cudaGetLastError();
 }

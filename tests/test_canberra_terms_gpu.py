@@ -1,8 +1,27 @@
-"""Canberra's division route against its shared reciprocals."""
+"""Canberra of few coordinates: every term a subtraction, an addition and a division, the
+sum d - 1 additions more, each rounded once (2^-24 relative of a sum of positive
+terms)."""
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("d", [1, 2, 3, 7])
+@pytest.mark.parametrize("layout", ["full", "dist"])
+def test_roundings_of_few_coordinates(gpu, rng, d, layout):
+    import torch
+    import gputools_gb300 as g
+    n = 700
+    P = np.exp(rng.standard_normal((n, d))).astype(np.float32)
+    got = g.distances_device(torch.from_numpy(P).cuda(), "canberra", layout=layout).cpu().numpy()
+    A = P.astype(np.float64)
+    want = sum(np.abs(A[:, None, k] - A[None, :, k]) / (A[:, None, k] + A[None, :, k])
+               for k in range(d))
+    i, j = np.triu_indices(n, 1)
+    got = got.reshape(n, n)[i, j] if layout == "full" else got
+    want = want[i, j]
+    assert np.all(np.abs(got - want) <= (d + 2) * 1.0001 * 2.0 ** -24 * want)
 
 
 @pytest.mark.parametrize("scale", [2.0 ** -40, 2.0 ** 70])
