@@ -66,6 +66,10 @@ enum WsSlot {
 };
 // Device buffer of at least `bytes` for `slot` on the current device.
 int ws_get(int slot, size_t bytes, void **ptr);
+// The same for scratch that a caller can do without (work on `s` would use it):
+// false, and no error left, if it cannot be had, or if `s` is being captured and the
+// slot would have to grow (an allocation would invalidate the capture).
+bool ws_try(int slot, size_t bytes, cudaStream_t s, void **ptr);
 void ws_release_all();
 // Page-locked host buffer of at least `bytes` for the current device
 // (grow-only, kept across calls, released with the device workspace).

@@ -254,8 +254,10 @@ int pearson_impl(int use, const float *dA, int64_t nA, const float *dB, int64_t 
     po.gate = nan_flag;
   }
   if (use == GT_EVERYTHING && path == GT_GRAM_TC_F16X3 && n > 0 &&
-      pearson_fma_wins(nA, nB, n, symmetric))
-    return pearson_fma(dA, nA, dB, nB, n, po, s);
+      pearson_fma_wins(nA, nB, n, symmetric)) {
+    int status = GT_OK;
+    if (pearson_fma(dA, nA, dB, nB, n, po, s, &status)) return status;
+  }
   if (tc) {
     void *zA = nullptr, *zB = nullptr;
     int64_t kpad = 0;

@@ -593,7 +593,7 @@ int pearson_exact(const void *zA, int64_t nA, const void *zB, int64_t nB, int64_
   const int pieces = k_pieces(ts.ntiles, kpad / kXBK, 16);
   void *P = nullptr;
   if (pieces > 1) {
-    if (ws_get(WS_PARTS, size_t(pieces) * 3 * size_t(nA) * size_t(nB) * 4, &P) == GT_OK) {
+    if (ws_try(WS_PARTS, size_t(pieces) * 3 * size_t(nA) * size_t(nB) * 4, s, &P)) {
       ExactPieces w;
       GT_TRY(tc_plane_map(&w.ma, zA, nA, kpad, kXPlanes, kBM, kXBK, true));
       GT_TRY(tc_plane_map(&w.mb, zB, nB, kpad, kXPlanes, kXB, kXBK, true));
@@ -610,8 +610,7 @@ int pearson_exact(const void *zA, int64_t nA, const void *zB, int64_t nB, int64_
       GT_CUDA(cudaGetLastError());
       return GT_OK;
     }
-    clear_error();  // no room for the pieces: in one
-  }
+  }  // without room for the pieces: in one
   using W = SingleWork<PearsonFinish>;
   W w;
   GT_TRY(tc_plane_map(&w.ma, zA, nA, kpad, kXPlanes, kBM, kXBK, true));

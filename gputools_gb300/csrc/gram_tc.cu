@@ -1579,10 +1579,8 @@ bool pearson_split(const void *zA, int64_t nA, const void *zB, int64_t nB, int64
   w.nk_total = nk;
   w.nk_part = cdiv(nk, int64_t(w.parts));
   void *P = nullptr;
-  if (ws_get(WS_PARTS, size_t(w.parts) * size_t(nA) * size_t(nB) * 4, &P) != GT_OK) {
-    clear_error();  // no room for the pieces: in one
-    return false;
-  }
+  if (!ws_try(WS_PARTS, size_t(w.parts) * size_t(nA) * size_t(nB) * 4, s, &P))
+    return false;  // no room for the pieces: in one
   w.part_stride = nA * nB;
   w.fin = StoreFinish{static_cast<float *>(P), nB, nA, nB};
   w.gate = fin.gate;

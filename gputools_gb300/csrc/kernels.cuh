@@ -67,8 +67,9 @@ int pearson_tc(const void *d_zA, int64_t nA, const void *d_zB, int64_t nB, int64
 
 // pearson_fma.cu: small "everything" problems on CUDA cores, statistics included.
 bool pearson_fma_wins(int64_t nA, int64_t nB, int64_t n, int symmetric);
-int pearson_fma(const float *dA, int64_t nA, const float *dB, int64_t nB, int64_t n,
-                const PearsonOut &out, cudaStream_t s);
+// False, with nothing done, where its scratch cannot be had.
+bool pearson_fma(const float *dA, int64_t nA, const float *dB, int64_t nB, int64_t n,
+                 const PearsonOut &out, cudaStream_t s, int *status);
 
 // gram_exact.cu: the error-free Pearson Gram (GT_GRAM_TC_F16X6): the
 // prologue writes three fixed-point fp16 digit planes per variable

@@ -171,11 +171,11 @@ bool pearson_fma_wins(int64_t nA, int64_t nB, int64_t n, int symmetric) {
   return n <= (symmetric ? 1500 : 2000) && entries <= 2.5e6 && entries * double(n) <= 2.4e8;
 }
 
-int pearson_fma(const float *dA, int64_t nA, const float *dB, int64_t nB, int64_t n,
-                const PearsonOut &out, cudaStream_t s) {
+bool pearson_fma(const float *dA, int64_t nA, const float *dB, int64_t nB, int64_t n,
+                 const PearsonOut &out, cudaStream_t s, int *status) {
   const int64_t ldz = cdiv(n, kFmaK) * kFmaK, nvar = nA + (out.symmetric ? 0 : nB);
   void *pz = nullptr;
-  GT_TRY(ws_get(WS_SCRATCH0, size_t(nvar) * size_t(ldz) * 4, &pz));
+  if (!ws_try(WS_SCRATCH0, size_t(nvar) * size_t(ldz) * 4, s, &pz)) return false;
   auto *Z = static_cast<float *>(pz);
   {
     ProfScope prof("pearson_prologue", s);
@@ -190,8 +190,11 @@ int pearson_fma(const float *dA, int64_t nA, const float *dB, int64_t nB, int64_
   pearson_fma_kernel<<<unsigned(cdiv(nB, kFmaTile) * cdiv(nA, kFmaTile)), kFmaThreads, 0, s>>>(
       Z, ZB, ldz, fin);
   count_launch();
-  GT_CUDA(cudaGetLastError());
-  return GT_OK;
+  *status = [&]() -> int {
+    GT_CUDA(cudaGetLastError());
+    return GT_OK;
+  }();
+  return true;
 }
 
 }  // namespace gt

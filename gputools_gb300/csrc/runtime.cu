@@ -232,6 +232,23 @@ int ws_get(int slot, size_t bytes, void **ptr) {
   return GT_OK;
 }
 
+bool ws_try(int slot, size_t bytes, cudaStream_t s, void **ptr) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess) cudaGetLastError();
+  if (cap != cudaStreamCaptureStatusNone) {
+    int dev = 0;
+    if (slot < 0 || slot >= WS_NSLOTS || current_device(&dev) != GT_OK) return false;
+    std::lock_guard<std::mutex> lk(g_mu);
+    const DeviceState &d = g_dev[dev];
+    if (!d.slot[slot] || d.bytes[slot] < bytes) return false;
+    *ptr = d.slot[slot];
+    return true;
+  }
+  if (ws_get(slot, bytes, ptr) == GT_OK) return true;
+  clear_error();
+  return false;
+}
+
 int host_ws_get(size_t bytes, void **ptr) {
   int dev = 0;
   GT_TRY(current_device(&dev));

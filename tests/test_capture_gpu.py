@@ -1,0 +1,83 @@
+"""Calls captured into a CUDA graph when the workspace has only what other calls left in
+it: scratch that a call can do without must not be allocated then (the capture would be
+invalid).  The replayed results are those of the same call made directly."""
+import ctypes
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+GT_OK = 0
+vp = lambda t: ctypes.c_void_p(t.data_ptr()) if t is not None else None
+
+
+def stream():
+    import torch
+    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+
+def replayed(gpu, warm, call, outputs):
+    """The outputs of `call` captured after a release of the workspace and `warm`, and
+    of the same call made directly."""
+    import torch
+    gpu.gt_release_workspace()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        if warm:
+            assert warm() == GT_OK, gpu.gt_last_error().decode()
+        assert gpu.gt_device_status(stream()) == GT_OK
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        status = call()
+    assert status == GT_OK, gpu.gt_last_error().decode()
+    for o in outputs:
+        o.fill_(-7.0)
+    graph.replay()
+    torch.cuda.synchronize()
+    got = [o.clone() for o in outputs]
+    for o in outputs:
+        o.fill_(-7.0)
+    assert call() == GT_OK, gpu.gt_last_error().decode()
+    assert gpu.gt_device_status(stream()) == GT_OK
+    return got, outputs
+
+
+def values(*shape, seed=1):
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    return torch.randn(shape, generator=gen, device="cuda")
+
+
+def pearson(gpu, A, B, out):
+    n = A.shape[1]
+    return lambda: gpu.gt_pmcc_device(0, vp(A), A.shape[0], vp(B), B.shape[0], n, None, vp(out),
+                                      None, stream())
+
+
+@pytest.mark.parametrize("path", ["f16x3", "f16x6"])
+def test_pearson_in_pieces(gpu, path):
+    """Few tiles of many observations after a problem of many tiles."""
+    import torch
+    import gputools_gb300 as g
+    big, few = values(3000, 2048), values(700, 2048, seed=2)
+    bout, out = torch.empty(3000, 3000, device="cuda"), torch.empty(700, 700, device="cuda")
+    old = g.get_gram_path()
+    g.set_gram_path(path)
+    try:
+        got, want = replayed(gpu, pearson(gpu, big, big, bout), pearson(gpu, few, few, out), [out])
+    finally:
+        g.set_gram_path(old)
+    # both within the path's tolerance (the sums are cut differently)
+    assert float((got[0] - want[0]).abs().max()) <= (3e-7 if path == "f16x6" else 2.2e-5)
+
+
+def test_small_pearson_of_two_sets(gpu):
+    """Both sets' rows go to one buffer, which is too small for the two."""
+    import torch
+    A0, B0 = values(200, 1000), values(20000, 1000)
+    A, B = values(300, 700, seed=2), values(1000, 700, seed=3)
+    o0, out = torch.empty(200, 20000, device="cuda"), torch.empty(300, 1000, device="cuda")
+    got, want = replayed(gpu, pearson(gpu, A0, B0, o0), pearson(gpu, A, B, out), [out])
+    assert float((got[0] - want[0]).abs().max()) <= 1.3e-5
