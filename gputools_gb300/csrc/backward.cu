@@ -1301,21 +1301,29 @@ int64_t dist_pairs_bytes(int64_t n, int64_t dim) {
   return nb * (nb + 1) / 2 * kPtT * (dim + 1) * 4;
 }
 
+// False, with nothing done, where its scratch cannot be had.
 template <int DMAX, int MODE>
-int dist_backward_pairs(const float *X, int64_t n, int64_t dim, const float *aux, float *dX,
-                        double *loss, cudaStream_t s) {
+bool dist_backward_pairs(const float *X, int64_t n, int64_t dim, const float *aux, float *dX,
+                         double *loss, cudaStream_t s, int *status) {
   using L = PtSmem<DMAX>;
-  auto kern = dist_pairs_kernel<DMAX, MODE>;
-  GT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::BYTES));
-  int per = 0;
-  GT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, kPtThreads, L::BYTES));
-  const int64_t slots = int64_t(sm_count()) * (per < 1 ? 1 : per);
+  void *pc = nullptr;
+  // the largest buffer first: the ordered kernel's fits where it does not
+  if (!ws_try(WS_SCRATCH0, size_t(dist_pairs_bytes(n, dim)), s, &pc)) return false;
   const int64_t nb = cdiv(n, kPtT), total = nb * (nb + 1) / 2;
+  auto kern = dist_pairs_kernel<DMAX, MODE>;
+  int per = 0;
+  *status = [&]() -> int {
+    GT_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::BYTES));
+    GT_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, kPtThreads, L::BYTES));
+    return GT_OK;
+  }();
+  if (*status != GT_OK) return true;
+  const int64_t slots = int64_t(sm_count()) * (per < 1 ? 1 : per);
   const int64_t len = cdiv(total, slots), segs = cdiv(total, len);
-  void *pc = nullptr, *pr = nullptr, *pl = nullptr;
-  GT_TRY(ws_get(WS_SCRATCH0, size_t(dist_pairs_bytes(n, dim)), &pc));
-  GT_TRY(ws_get(WS_SCRATCH1, size_t(segs + nb) * kPtT * size_t(dim + 1) * 4, &pr));
-  GT_TRY(ws_get(WS_SCRATCH2, size_t(segs) * 8, &pl));
+  void *pr = nullptr, *pl = nullptr;
+  if (!ws_try(WS_SCRATCH1, size_t(segs + nb) * kPtT * size_t(dim + 1) * 4, s, &pr) ||
+      !ws_try(WS_SCRATCH2, size_t(segs) * 8, s, &pl))
+    return false;
   PtPartials pp;
   pp.col = static_cast<float *>(pc);
   pp.colw = pp.col + total * kPtT * dim;
@@ -1330,8 +1338,11 @@ int dist_backward_pairs(const float *X, int64_t n, int64_t dim, const float *aux
     loss_reduce_kernel<<<1, kLossThreads, 0, s>>>(pp.loss, segs, loss);
     count_launch();
   }
-  GT_CUDA(cudaGetLastError());
-  return GT_OK;
+  *status = [&]() -> int {
+    GT_CUDA(cudaGetLastError());
+    return GT_OK;
+  }();
+  return true;
 }
 
 template <int MODE>
@@ -1344,11 +1355,14 @@ int launch_dist_backward(const float *X, int64_t n, int64_t dim, const float *au
   // 8192 x 48 500 / 790 / 671, 10000 x 40 720 / - / 1090.  Past that the ordered
   // kernel holds no n^2 workspace; above 32 dimensions and up to 32768 points
   // (11 GB there) the tensor-core form is 10-15 % faster than it, and above 64
-  // dimensions it is the only one.
+  // dimensions it is the only one.  They also take the problems whose partial sums
+  // the device has no room for.
   if (dim <= 64 && dist_pairs_bytes(n, dim) <= (int64_t(1) << 30)) {
-    if (dim <= 16) return dist_backward_pairs<16, MODE>(X, n, dim, aux, dX, loss, s);
-    if (dim <= 32) return dist_backward_pairs<32, MODE>(X, n, dim, aux, dX, loss, s);
-    return dist_backward_pairs<64, MODE>(X, n, dim, aux, dX, loss, s);
+    int status = GT_OK;
+    if (dim <= 16   ? dist_backward_pairs<16, MODE>(X, n, dim, aux, dX, loss, s, &status)
+        : dim <= 32 ? dist_backward_pairs<32, MODE>(X, n, dim, aux, dX, loss, s, &status)
+                    : dist_backward_pairs<64, MODE>(X, n, dim, aux, dX, loss, s, &status))
+      return status;
   }
   if (dim > 64 || (dim > 32 && n >= 8192 && n <= 32768))
     return dist_backward_tc<MODE>(X, n, dim, aux, dX, loss, s);

@@ -81,3 +81,24 @@ def test_small_pearson_of_two_sets(gpu):
     o0, out = torch.empty(200, 20000, device="cuda"), torch.empty(300, 1000, device="cuda")
     got, want = replayed(gpu, pearson(gpu, A0, B0, o0), pearson(gpu, A, B, out), [out])
     assert float((got[0] - want[0]).abs().max()) <= 1.3e-5
+
+
+@pytest.mark.parametrize("mds", [True, False])
+def test_distance_adjoint(gpu, mds):
+    """20000 points of 16 dimensions: 213 MB of partial sums where 25 MB are at hand.  Both
+    kernels sum 20000 terms in float, in another order: 2e-5 of the largest entry."""
+    import torch
+    n, d = 20000, 16
+    Z, zo = values(4000, 1500), torch.empty(4000, 4000, device="cuda")
+    X, out = values(n, d, seed=2), torch.empty(n, d, device="cuda")
+    loss = torch.empty(1, dtype=torch.float64, device="cuda")
+    if mds:
+        aux = torch.rand(n * (n - 1) // 2, device="cuda") + 4.0
+        call = lambda: gpu.gt_mds_stress_device(vp(X), n, d, vp(aux), vp(out), vp(loss), stream())
+    else:
+        aux = values(n, n, seed=3)
+        call = lambda: gpu.gt_dist_backward_device(vp(X), n, d, vp(aux), vp(out), stream())
+    got, want = replayed(gpu, pearson(gpu, Z, Z.clone(), zo), call, [out, loss])
+    assert float((got[0] - want[0]).abs().max()) <= 2e-5 * float(want[0].abs().max())
+    if mds:
+        assert abs(float(got[1] - want[1])) <= 1e-6 * float(want[1])
