@@ -439,9 +439,13 @@ int kendall_impl(const float *dX, int64_t nx, const float *dY, int64_t ny, int64
   GT_CUDA(cudaMemsetAsync(S, 0, bytes, s));
 
   if (Dr > 0) {
-    const SignPlan big = make_sign_plan(n, rows_chunk);
+    // ... or as many as the device has room for (four times the bytes of the bit masks
+    // that batches count)
     void *pP = nullptr;
-    GT_TRY(ws_get(WS_SCRATCH2, size_t(nvar) * size_t(big.kpad), &pP));
+    while (rows_chunk > 1 &&
+           !ws_try(WS_SCRATCH2, size_t(nvar) * size_t(make_sign_plan(n, rows_chunk).kpad), s, &pP))
+      rows_chunk = cdiv(rows_chunk, 2);
+    if (!pP) GT_TRY(ws_get(WS_SCRATCH2, size_t(nvar) * size_t(make_sign_plan(n, 1).kpad), &pP));
     auto *P = static_cast<uint8_t *>(pP);
     tc::WaitCfg wc;
     GT_TRY(make_wait_cfg(&wc));

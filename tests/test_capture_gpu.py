@@ -102,3 +102,16 @@ def test_distance_adjoint(gpu, mds):
     assert float((got[0] - want[0]).abs().max()) <= 2e-5 * float(want[0].abs().max())
     if mds:
         assert abs(float(got[1] - want[1])) <= 1e-6 * float(want[1])
+
+
+def test_kendall(gpu):
+    """100 MB of signs where 34 are at hand: more passes, the same integers."""
+    import torch
+    n = 1000
+    X0, X = values(60, n), values(200, n, seed=2)
+    o0 = torch.empty(60, 60, dtype=torch.float64, device="cuda")
+    out = torch.empty(200, 200, dtype=torch.float64, device="cuda")
+    call = lambda X, o: lambda: gpu.gt_kendall_device(vp(X), X.shape[0], vp(X), X.shape[0], n,
+                                                      vp(o), stream())
+    got, want = replayed(gpu, call(X0, o0), call(X, out), [out])
+    assert torch.equal(got[0], want[0])
