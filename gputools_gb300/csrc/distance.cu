@@ -236,11 +236,21 @@ __device__ __forceinline__ bool canberra_prepare(float4 (&r)[CHUNKS], unsigned &
   return bad;
 }
 
-// bits[i * words + w]: the nonzero pattern of point i (pack_nonzero_kernel).
+// Word w of a point's nonzero pattern, from the point itself.
+__device__ __forceinline__ unsigned canberra_scan(const float *p, int64_t w, int64_t K) {
+  unsigned b = 0;
+#pragma unroll 1
+  for (int64_t k = 32 * w; k < K && k < 32 * w + 32; k++)
+    b |= unsigned(__ldg(p + k) != 0.f) << (k & 31);
+  return b;
+}
+
+// bits[i * words + w]: the nonzero pattern of point i (pack_nonzero_kernel); without BITS,
+// where the device has no room for it, the points are read again at the end.
 // 64 x 64 tiles, three blocks an SM: 128 x 128 tiles with two blocks or one
 // measured 1.51 and 1.87 ms where these took 1.49, and 215 / 236 us against 185
 // at 4000 x 100 (full).
-template <bool FEW>
+template <bool FEW, bool BITS>
 __global__ void __launch_bounds__(kSimtThreads, 3)
 canberra_kernel(SimtArgs a, const unsigned *__restrict__ bits, int64_t words,
                 OutDist<OpValue> out) {
@@ -400,6 +410,10 @@ canberra_kernel(SimtArgs a, const unsigned *__restrict__ bits, int64_t words,
 
   // coordinates where both points are zero: all but those nonzero in either
   // (the words' bits past dim are zero in both)
+  auto word = [&](const float *p, int64_t i, int64_t w) {
+    if constexpr (BITS) return bits[i * words + w];
+    else return canberra_scan(p, w, a.K);
+  };
   float val[TM][TN][1];
   int used[TM][TN];
 #pragma unroll
@@ -411,12 +425,12 @@ canberra_kernel(SimtArgs a, const unsigned *__restrict__ bits, int64_t words,
 #pragma unroll
     for (int j = 0; j < TN; j++) {
       const int64_t c = col0 + tx + 16 * j;
-      zb[j] = c < a.nc ? bits[c * words + w] : 0u;
+      zb[j] = c < a.nc ? word(a.C + c * a.ldc, c, w) : 0u;
     }
 #pragma unroll
     for (int i = 0; i < TM; i++) {
       const int64_t r = row0 + simt_row(i, ty);
-      const unsigned za = r < a.nr ? bits[r * words + w] : 0u;
+      const unsigned za = r < a.nr ? word(a.R + r * a.ldr, r, w) : 0u;
 #pragma unroll
       for (int j = 0; j < TN; j++) used[i][j] += __popc(za | zb[j]);
     }
@@ -448,10 +462,10 @@ cudaError_t run_canberra(const float *pts, const unsigned *bits, int64_t n, int6
   const SimtArgs a = dist_args(pts, n, dim);
   const OutDist<OpValue> o{OpValue{}, out, n, dim, layout};
   const unsigned g = unsigned(cdiv(n, 64));
-  if (dim < kCanMinK)
-    canberra_kernel<true><<<dim3(g, g), kSimtThreads, 0, st>>>(a, bits, cdiv(dim, 32), o);
-  else
-    canberra_kernel<false><<<dim3(g, g), kSimtThreads, 0, st>>>(a, bits, cdiv(dim, 32), o);
+  const bool few = dim < kCanMinK;
+  auto kern = bits ? (few ? canberra_kernel<true, true> : canberra_kernel<false, true>)
+                   : (few ? canberra_kernel<true, false> : canberra_kernel<false, false>);
+  kern<<<dim3(g, g), kSimtThreads, 0, st>>>(a, bits, cdiv(dim, 32), o);
   count_launch();
   return cudaGetLastError();
 }
@@ -493,12 +507,16 @@ int dist_simt(const float *d_pts, int64_t n, int64_t dim, float *d_out, int layo
   case GT_CANBERRA:
   case GT_BINARY: {
     const int64_t words = cdiv(dim, 32);
+    const size_t bytes = size_t(n) * size_t(words) * 4;
     void *pb = nullptr;
-    GT_TRY(ws_get(WS_SCRATCH0, size_t(n) * size_t(words) * 4, &pb));
+    if (method == GT_BINARY) GT_TRY(ws_get(WS_SCRATCH0, bytes, &pb));
+    else if (!ws_try(WS_SCRATCH0, bytes, st, &pb)) pb = nullptr;
     auto *bits = static_cast<unsigned *>(pb);
-    pack_nonzero_kernel<<<unsigned(cdiv(n, 8)), 256, 0, st>>>(d_pts, n, dim, words, bits);
-    count_launch();
-    e = cudaGetLastError();
+    if (bits) {
+      pack_nonzero_kernel<<<unsigned(cdiv(n, 8)), 256, 0, st>>>(d_pts, n, dim, words, bits);
+      count_launch();
+      e = cudaGetLastError();
+    }
     if (e != cudaSuccess) break;
     if (method == GT_CANBERRA) {
       e = run_canberra(d_pts, bits, n, dim, d_out, layout, st);

@@ -115,3 +115,14 @@ def test_kendall(gpu):
                                                       vp(o), stream())
     got, want = replayed(gpu, call(X0, o0), call(X, out), [out])
     assert torch.equal(got[0], want[0])
+
+
+@pytest.mark.parametrize("n,d", [(300, 5), (200, 70)])
+def test_canberra_as_the_first_call(gpu, n, d):
+    import torch
+    P = values(n, d).abs()
+    P[torch.rand(n, d, device="cuda") < 0.3] = 0
+    out = torch.empty(n, n, device="cuda")
+    call = lambda: gpu.gt_distances_device(vp(P), n, d, vp(out), 0, 3, ctypes.c_float(2.0), stream())
+    got, want = replayed(gpu, None, call, [out])
+    assert torch.equal(got[0].view(torch.int32), want[0].view(torch.int32))
