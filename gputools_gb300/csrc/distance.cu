@@ -194,7 +194,9 @@ struct OpValue {
 // values make a zero product, whose reciprocal gives the term's +Inf, or NaN
 // where both terms are infinite (0 times Inf): nothing else makes a NaN there,
 // so it is read as +Inf.  Coordinates where both points are zero are counted
-// at the end from the points' packed nonzero bits, 32 to a popcount.  From the
+// at the end from the points' nonzero bits, 32 to a popcount, which the slabs leave in
+// shared memory (a buffer in the workspace, filled by a launch of its own, made calls on
+// two streams share it).  From the
 // first slab with a huge, tiny or non-finite value on (voted by the barrier
 // that ends the slab before it) a tile takes the divisions, on the values
 // themselves.  Fewer than 8 coordinates (FEW), whose additions do not make up for the
@@ -204,6 +206,7 @@ struct OpValue {
 // before, 4.4 of them the two FP64 divisions of each rescaled entry).
 constexpr float kCanZero = 0x1p-60f, kCanLo = 0x1p-30f, kCanHi = 0x1p60f;
 constexpr int kCanMinK = 8;
+constexpr int kCanSlabs = 32;  // slabs whose bits the shared memory holds
 
 // sum * dim / used with one rounding (the product's and the quotient's
 // residuals are added back) where the product cannot overflow.
@@ -217,43 +220,31 @@ __device__ __forceinline__ float canberra_finish(float sum, int zeros, int64_t K
   return q + __fdividef(fmaf(-q, used, p) + pe, used);
 }
 
-// Replaces a chunk's zeros (noted in the next bits of `zeros`); whether a value is out
-// of the range.
-template <int CHUNKS>
-__device__ __forceinline__ bool canberra_prepare(float4 (&r)[CHUNKS], unsigned &zeros) {
+// The nonzero bits of a chunk.
+__device__ __forceinline__ unsigned canberra_bits(const float4 &v) {
+  return unsigned(v.x != 0.f) | unsigned(v.y != 0.f) << 1 | unsigned(v.z != 0.f) << 2 |
+         unsigned(v.w != 0.f) << 3;
+}
+
+// Replaces a chunk's zeros; whether a value is out of the range.
+__device__ __forceinline__ bool canberra_prepare(float4 &v) {
   bool bad = false;
+  float *e = &v.x;
 #pragma unroll
-  for (int s = 0; s < CHUNKS; s++) {
-    float *e = &r[s].x;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const bool zero = e[i] == 0.f;
-      bad |= !(zero || (fabsf(e[i]) >= kCanLo && fabsf(e[i]) <= kCanHi));
-      if (zero) e[i] = kCanZero;
-      zeros = 2 * zeros + zero;
-    }
+  for (int i = 0; i < 4; i++) {
+    const bool zero = e[i] == 0.f;
+    bad |= !(zero || (fabsf(e[i]) >= kCanLo && fabsf(e[i]) <= kCanHi));
+    if (zero) e[i] = kCanZero;
   }
   return bad;
 }
 
-// Word w of a point's nonzero pattern, from the point itself.
-__device__ __forceinline__ unsigned canberra_scan(const float *p, int64_t w, int64_t K) {
-  unsigned b = 0;
-#pragma unroll 1
-  for (int64_t k = 32 * w; k < K && k < 32 * w + 32; k++)
-    b |= unsigned(__ldg(p + k) != 0.f) << (k & 31);
-  return b;
-}
-
-// bits[i * words + w]: the nonzero pattern of point i (pack_nonzero_kernel); without BITS,
-// where the device has no room for it, the points are read again at the end.
 // 64 x 64 tiles, three blocks an SM: 128 x 128 tiles with two blocks or one
 // measured 1.51 and 1.87 ms where these took 1.49, and 215 / 236 us against 185
 // at 4000 x 100 (full).
-template <bool FEW, bool BITS>
+template <bool FEW>
 __global__ void __launch_bounds__(kSimtThreads, 3)
-canberra_kernel(SimtArgs a, const unsigned *__restrict__ bits, int64_t words,
-                OutDist<OpValue> out) {
+canberra_kernel(SimtArgs a, OutDist<OpValue> out) {
   constexpr int TM = 4, TN = 4, BM = 16 * TM, BN = 16 * TN;
   constexpr int LDA = simt_ld<BM>(), LDB = simt_ld<BN>();
   const int ti = blockIdx.y, tj = blockIdx.x;
@@ -261,6 +252,9 @@ canberra_kernel(SimtArgs a, const unsigned *__restrict__ bits, int64_t words,
   const int64_t row0 = int64_t(ti) * BM, col0 = int64_t(tj) * BN;
   __shared__ __align__(16) float sA[2][kSimtBK * LDA];
   __shared__ __align__(16) float sB[2][kSimtBK * LDB];
+  // nonzero bits of rows and columns, 16 coordinates each (one slab); rows an odd number
+  // of words apart
+  __shared__ __align__(4) uint16_t nz[2][64][kCanSlabs + 2];
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
 
   float2 acc[TM][TN / 2];
@@ -271,20 +265,29 @@ canberra_kernel(SimtArgs a, const unsigned *__restrict__ bits, int64_t words,
   float4 ra[BM * 4 / kSimtThreads], rb[BN * 4 / kSimtThreads];
   simt_load<BM, OpEuclid>(ra, a.R, a.ldr, a.nr, row0, 0, a.K, a.vec_ok);
   simt_load<BN, OpEuclid>(rb, a.C, a.ldc, a.nc, col0, 0, a.K, a.vec_ok);
-  // The slab in ra, rb to buffer b, its zeros replaced; true if a value is out of the
-  // range (uniform): then the slab is stored as it is.
-  auto store = [&](int b) {
-    unsigned zeros = 0;
-    bool bad = canberra_prepare(ra, zeros);
-    bad |= canberra_prepare(rb, zeros);
+  static_assert(BM * 4 == kSimtThreads && BN * 4 == kSimtThreads, "a chunk a thread");
+  auto note = [&](int kb) {  // the bits of slab kb, in ra and rb: four threads' chunks a row
+    const int q = threadIdx.x & 3;
+    unsigned m = (canberra_bits(ra[0]) | canberra_bits(rb[0]) << 16) << (4 * q);
+    m |= __shfl_xor_sync(0xffffffffu, m, 1);
+    m |= __shfl_xor_sync(0xffffffffu, m, 2);
+    if (q < 2 && kb < kCanSlabs) nz[q][threadIdx.x >> 2][kb] = uint16_t(q ? m >> 16 : m);
+    return m;
+  };
+  // Slab kb in ra, rb to its buffer, zeros replaced; true if a value is out of the range
+  // (uniform): then the slab is stored as it is.
+  auto store = [&](int kb) {
+    const int b = kb & 1, q = 4 * (threadIdx.x & 3);
+    const unsigned m = note(kb);
+    bool bad = canberra_prepare(ra[0]);
+    bad |= canberra_prepare(rb[0]);
     simt_store<BM, false>(sA[b], ra);
     simt_store<BN, true>(sB[b], rb);
     if (!__syncthreads_or(bad)) return false;
-    static_assert(BM * 4 == kSimtThreads && BN * 4 == kSimtThreads, "a chunk a thread");
 #pragma unroll
     for (int i = 0; i < 4; i++) {
-      if ((zeros >> (7 - i)) & 1u) (&ra[0].x)[i] = 0.f;
-      if ((zeros >> (3 - i)) & 1u) (&rb[0].x)[i] = 0.f;
+      if (!((m >> (q + i)) & 1u)) (&ra[0].x)[i] = 0.f;
+      if (!((m >> (q + i + 16)) & 1u)) (&rb[0].x)[i] = 0.f;
     }
     simt_store<BM, false>(sA[b], ra);
     simt_store<BN, true>(sB[b], rb);
@@ -364,7 +367,7 @@ canberra_kernel(SimtArgs a, const unsigned *__restrict__ bits, int64_t words,
         }
       }
     }
-    if (more) divide = store(buf ^ 1);
+    if (more) divide = store(kb + 1);
     else __syncthreads();
   }
 #pragma unroll
@@ -402,38 +405,51 @@ canberra_kernel(SimtArgs a, const unsigned *__restrict__ bits, int64_t words,
       }
     }
     if (more) {
+      note(kb + 1);
       simt_store<BM, false>(sA[buf ^ 1], ra);
       simt_store<BN, true>(sB[buf ^ 1], rb);
     }
     __syncthreads();
   }
 
-  // coordinates where both points are zero: all but those nonzero in either
-  // (the words' bits past dim are zero in both)
-  auto word = [&](const float *p, int64_t i, int64_t w) {
-    if constexpr (BITS) return bits[i * words + w];
-    else return canberra_scan(p, w, a.K);
-  };
+  // coordinates where both points are zero: all but those nonzero in either (the bits
+  // past dim are zero in both)
   float val[TM][TN][1];
   int used[TM][TN];
 #pragma unroll
   for (int i = 0; i < TM; i++)
 #pragma unroll
     for (int j = 0; j < TN; j++) used[i][j] = 0;
-  for (int64_t w = 0; w < words; w++) {
-    unsigned zb[TN];
+  for (int64_t k0 = 0;;) {  // slabs k0 / 16 .. in nz
+    const int64_t left = (a.K - k0 + kSimtBK - 1) / kSimtBK;
+    const int slabs = left < kCanSlabs ? int(left) : kCanSlabs;
+    for (int t = 0; t < slabs; t += 2) {
+      const unsigned in = t + 1 < slabs ? 0xffffffffu : 0xffffu;
+      unsigned zb[TN];
 #pragma unroll
-    for (int j = 0; j < TN; j++) {
-      const int64_t c = col0 + tx + 16 * j;
-      zb[j] = c < a.nc ? word(a.C + c * a.ldc, c, w) : 0u;
+      for (int j = 0; j < TN; j++)
+        zb[j] = *reinterpret_cast<const unsigned *>(&nz[1][tx + 16 * j][t]) & in;
+#pragma unroll
+      for (int i = 0; i < TM; i++) {
+        const unsigned za = *reinterpret_cast<const unsigned *>(&nz[0][simt_row(i, ty)][t]) & in;
+#pragma unroll
+        for (int j = 0; j < TN; j++) used[i][j] += __popc(za | zb[j]);
+      }
     }
-#pragma unroll
-    for (int i = 0; i < TM; i++) {
-      const int64_t r = row0 + simt_row(i, ty);
-      const unsigned za = r < a.nr ? word(a.R + r * a.ldr, r, w) : 0u;
-#pragma unroll
-      for (int j = 0; j < TN; j++) used[i][j] += __popc(za | zb[j]);
+    k0 += kCanSlabs * kSimtBK;
+    if (k0 >= a.K) break;
+    // further coordinates: from the points again
+    __syncthreads();
+#pragma unroll 1
+    for (int q = threadIdx.x >> 5; q < 128 * kCanSlabs / 2; q += kSimtThreads / 32) {
+      const int side = q >> 10, row = (q >> 4) & 63, t = 2 * (q & 15);
+      static_assert(kCanSlabs == 32, "sixteen words a row");
+      const int64_t i = (side ? col0 : row0) + row, k = k0 + 16 * t + (threadIdx.x & 31);
+      const bool on = i < a.nr && k < a.K && __ldg(a.R + i * a.ldr + k) != 0.f;
+      const unsigned w = __ballot_sync(0xffffffffu, on);
+      if ((threadIdx.x & 31) == 0) *reinterpret_cast<unsigned *>(&nz[side][row][t]) = w;
     }
+    __syncthreads();
   }
 #pragma unroll
   for (int i = 0; i < TM; i++)
@@ -456,16 +472,14 @@ SimtArgs dist_args(const float *pts, int64_t n, int64_t dim) {
   return a;
 }
 
-cudaError_t run_canberra(const float *pts, const unsigned *bits, int64_t n, int64_t dim,
-                         float *out, int layout, cudaStream_t st) {
+cudaError_t run_canberra(const float *pts, int64_t n, int64_t dim, float *out, int layout,
+                         cudaStream_t st) {
   ProfScope prof("dist", st);
   const SimtArgs a = dist_args(pts, n, dim);
   const OutDist<OpValue> o{OpValue{}, out, n, dim, layout};
   const unsigned g = unsigned(cdiv(n, 64));
-  const bool few = dim < kCanMinK;
-  auto kern = bits ? (few ? canberra_kernel<true, true> : canberra_kernel<false, true>)
-                   : (few ? canberra_kernel<true, false> : canberra_kernel<false, false>);
-  kern<<<dim3(g, g), kSimtThreads, 0, st>>>(a, bits, cdiv(dim, 32), o);
+  auto kern = dim < kCanMinK ? canberra_kernel<true> : canberra_kernel<false>;
+  kern<<<dim3(g, g), kSimtThreads, 0, st>>>(a, o);
   count_launch();
   return cudaGetLastError();
 }
@@ -504,26 +518,19 @@ int dist_simt(const float *d_pts, int64_t n, int64_t dim, float *d_out, int layo
   case GT_EUCLIDEAN: e = run_metric(OpEuclid{}, d_pts, n, dim, d_out, layout, st); break;
   case GT_MAXIMUM: e = run_metric(OpMaximum{}, d_pts, n, dim, d_out, layout, st); break;
   case GT_MANHATTAN: e = run_metric(OpManhattan{}, d_pts, n, dim, d_out, layout, st); break;
-  case GT_CANBERRA:
+  case GT_CANBERRA: e = run_canberra(d_pts, n, dim, d_out, layout, st); break;
   case GT_BINARY: {
     const int64_t words = cdiv(dim, 32);
-    const size_t bytes = size_t(n) * size_t(words) * 4;
     void *pb = nullptr;
-    if (method == GT_BINARY) GT_TRY(ws_get(WS_SCRATCH0, bytes, &pb));
-    else if (!ws_try(WS_SCRATCH0, bytes, st, &pb)) pb = nullptr;
-    auto *bits = static_cast<unsigned *>(pb);
-    if (bits) {
-      pack_nonzero_kernel<<<unsigned(cdiv(n, 8)), 256, 0, st>>>(d_pts, n, dim, words, bits);
-      count_launch();
-      e = cudaGetLastError();
-    }
-    if (e != cudaSuccess) break;
-    if (method == GT_CANBERRA) {
-      e = run_canberra(d_pts, bits, n, dim, d_out, layout, st);
-    } else {
-      const float *fbits = static_cast<const float *>(pb);
-      e = dim < 65536 ? run_metric(OpBinaryPacked{}, fbits, n, words, d_out, layout, st)
-                      : run_metric(OpBinaryBits{}, fbits, n, words, d_out, layout, st);
+    GT_TRY(ws_get(WS_SCRATCH0, size_t(n) * size_t(words) * 4, &pb));
+    pack_nonzero_kernel<<<unsigned(cdiv(n, 8)), 256, 0, st>>>(d_pts, n, dim, words,
+                                                             static_cast<unsigned *>(pb));
+    count_launch();
+    e = cudaGetLastError();
+    if (e == cudaSuccess) {
+      const float *bits = static_cast<const float *>(pb);
+      e = dim < 65536 ? run_metric(OpBinaryPacked{}, bits, n, words, d_out, layout, st)
+                      : run_metric(OpBinaryBits{}, bits, n, words, d_out, layout, st);
     }
     break;
   }
