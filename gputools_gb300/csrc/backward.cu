@@ -699,7 +699,7 @@ __global__ void dist_backward_reduce_kernel(const float *__restrict__ X, int64_t
 // segment ends, go to partial buffers that a second kernel adds in a fixed order.
 // Bound by issue and latency at 16 warps an SM (61 % of the issue slots): 185
 // instructions a pair, where the ordered kernel makes 380.  8192 x 32 (MDS stress):
-// 296 us per call, 455 with ordered pairs; the gradient's error 0.8e-7 (1.2e-7).
+// 299 us per call, 455 with ordered pairs; the gradient's error 0.8e-7 (1.2e-7).
 constexpr int kPtT = 64, kPtThreads = 256;
 
 template <int DMAX>
@@ -1351,8 +1351,8 @@ int launch_dist_backward(const float *X, int64_t n, int64_t dim, const float *au
   // Up to 64 dimensions each unordered pair once, while the partial sums take at
   // most 1 GB (about 33000 points at 32 dimensions, 23000 at 64).  Measured (MDS
   // stress, us, pairs / ordered pairs / tensor cores): 1000 x 32 24 / 34 / -,
-  // 4096 x 64 149 / 236 / 235, 8192 x 16 203 / 309 / -, 8192 x 32 296 / 455 / 670,
-  // 8192 x 48 500 / 790 / 671, 10000 x 40 720 / - / 1090.  Past that the ordered
+  // 4096 x 64 150 / 236 / 235, 8192 x 16 203 / 309 / -, 8192 x 32 299 / 455 / 670,
+  // 8192 x 48 507 / 790 / 671, 10000 x 40 720 / - / 1090.  Past that the ordered
   // kernel holds no n^2 workspace; above 32 dimensions and up to 32768 points
   // (11 GB there) the tensor-core form is 10-15 % faster than it, and above 64
   // dimensions it is the only one.  They also take the problems whose partial sums

@@ -202,8 +202,9 @@ struct OpValue {
 // themselves.  Fewer than 8 coordinates (FEW), whose additions do not make up for the
 // roundings of a shared denominator, take a reciprocal a term and correct the quotient
 // by its residual (about half an ulp, as the division).
-// Bound by the FMA pipe: 16000 x 64, a tenth zeros, dist layout: 1.53 ms (9.54
-// before, 4.4 of them the two FP64 divisions of each rescaled entry).
+// Bound by issue (68 % of the slots): 16000 x 64, a tenth zeros, dist layout: 1.55 ms
+// (9.54 before, 4.4 of them the two FP64 divisions of each rescaled entry); by divisions,
+// signed values of 1e-12, 4.6 (5.1).
 constexpr float kCanZero = 0x1p-60f, kCanLo = 0x1p-30f, kCanHi = 0x1p60f;
 constexpr int kCanMinK = 8;
 constexpr int kCanSlabs = 32;  // slabs whose bits the shared memory holds

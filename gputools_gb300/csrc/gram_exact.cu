@@ -35,10 +35,10 @@
 // lies wholly below the diagonal of a symmetric problem is skipped).  Problems
 // that fill the chip with 256 x 256 tiles run them on pairs of CTAs
 // (cta_group::2, clusters of two): the halves are 256 x 128, each CTA holding 128
-// rows of A and 64 of B, so a stage fetches a quarter less.  20000 x 4096: 5.9 ms
-// (1.66 PFLOP/s; cuBLAS holds 1.71 under the power limit), 6.7 on single CTAs
-// with one lane issuing from a branch.  With the operands left in place (no
-// copies) the MMAs alone take 4.7: the copies' latency bounds it.
+// rows of A and 64 of B, so a stage fetches a quarter less.  20000 x 4096: 5.4 to 5.8 ms
+// by the box (1.73 PFLOP/s at 5.67; cuBLAS holds 1.71 under the power limit), the call
+// 0.3 more; 6.7 the call on single CTAs with one lane issuing from a branch.  With the
+// operands left in place (no copies) the call takes 4.96: the copies' latency bounds it.
 //   warp 0      TMA producer: 3-D loads of the three digit planes of the A
 //               (128-row) and B (128- or 64-row) boxes, 32 k per stage;
 //   warp 1      allocates 512 TMEM columns (three 128 x 128 accumulators) and

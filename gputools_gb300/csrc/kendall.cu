@@ -141,7 +141,7 @@ size_t sign_smem(const SignPlan &p) {
 // one row segment and groups * dper pair rows.  Each thread keeps its four
 // x[i] in registers and slides a window of four x[i + d] along: one shared
 // read per four signs, conflict-free because the window is stored by its
-// index modulo 4.  Bound by the compares and selects of the ALU pipe (78 %
+// index modulo 4.  Bound by the compares and selects of the ALU pipe (87 %
 // busy); 500 x 1000: 61 us for 125 MB of signs.
 __global__ void __launch_bounds__(kSgThreads)
 kendall_signs_kernel(const float *__restrict__ X, int64_t nx, const float *__restrict__ Y,

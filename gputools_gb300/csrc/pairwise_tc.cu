@@ -373,7 +373,7 @@ pairwise_tc_kernel(const __grid_constant__ PairwiseArgs a, const tc::WaitCfg wc)
       // lanes on consecutive columns, rows r after transpose8 (eight columns of
       // four rows an instruction; one column of 32 rows, an eighth of each
       // sector, took a third of the kernel's time: 1000 observations of 4000
-      // variables 399 -> 306 us, 200 of 4000 240 -> 126).
+      // variables 399 -> 296 us, 200 of 4000 240 -> 116).
       const int64_t rbase = r - lane;
       const bool inner = c0 + 8 <= a.nc && rbase + 32 <= a.nr && (!a.symmetric || rbase + 31 < c0);
       auto put = [&](float *o, float (&v)[8]) {

@@ -2,11 +2,11 @@
 //
 // GB300's FP64 pipe runs at a small fraction of its FP32 pipe, so the sums
 // over observations are compensated float pairs (Knuth's TwoSum, squares with
-// their exact FMA residual), about 2^-44 relative, and so are the few
+// their exact FMA residual), about 2^-47 relative, and so are the few
 // operations that finish a variable's statistics: every lane of its warp makes
 // them, and the 60 or so that they took in FP64 (16 cycles of the SM's FP64 pipe
 // each) were most of the batched prologue (300 problems, 220000 variables:
-// 683 us, now 450; 330 with the lighter passes below).
+// 683 us, now 450; 348 with the lighter passes below).
 #pragma once
 
 #include <cuda_runtime.h>

@@ -160,9 +160,10 @@ void gt_release_workspace(void);
  * limit: a wait that gives up makes its CTA stop, drain its copies and
  * multiplies, free its tensor memory and set the device's error word, and
  * the call's results are then incomplete.  The host-buffer entries (gt_pmcc,
- * gt_distances, gt_mutual_info, the .C entries) read the word before they
- * return and report GT_ETIMEOUT.  Device-buffer entries and batch-plan
- * launches are asynchronous and report it only through gt_device_status:
+ * gt_distances, gt_kendall, gt_mutual_info, the .C entries) read the word before
+ * they return and report GT_ETIMEOUT.  Device-buffer entries (gt_pmcc_device,
+ * gt_distances_device, gt_kendall_device, gt_mutual_info_device, the adjoints) and
+ * batch-plan launches are asynchronous and report it only through gt_device_status:
  * it synchronises `stream`, returns GT_ETIMEOUT if any such kernel on the
  * current device timed out since the last check on that device (and clears
  * the word), else GT_OK. */
@@ -278,8 +279,8 @@ int gt_cor_backward_device(const float *d_X, int64_t p, int64_t n,
 /* dL/dX of the Euclidean distances D of the rows of X (n x dim row-major)
  * given G = dL/dD (n x n, G[i*n + j]); terms with D_ij = 0 contribute 0.
  * Up to 64 dimensions CUDA-core passes (D recomputed, nothing n x n stored):
- * each unordered pair once with up to 1 GB of partial sums, past that every
- * ordered pair, except 33..64 dimensions up to 32768 points; there and above 64
+ * each unordered pair once with up to 1 GB of partial sums, past that (or where the
+ * device has no room for them) every ordered pair, except 33..64 dimensions up to 32768 points; there and above 64
  * dimensions D from the tensor-core distance path, W = (G + G^T) / D as
  * split-bf16 planes and W X on the tensor cores (about 10 n^2 bytes of device
  * workspace). */
